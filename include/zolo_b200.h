@@ -16,7 +16,8 @@
  * INFO conventions follow the reference: 0 success, -i for a bad scalar
  * argument i, -(i*100+j) for entry j of array argument i, -12 / -16 for a
  * too-small LWORK / LWORK2 (pqdwhfacs.f90:286-294), > 0 from a factorisation.
- * GPU failures are reported as INFO = -1000 - cudaError_t.  Nothing aborts.
+ * GPU failures are reported as INFO = -1000 - cudaError_t, a bounded wait inside a kernel that
+ * timed out as INFO = -2000 - 9xx.  Nothing aborts.
  *
  * Threading: every handle owns one CUDA stream; calls on one handle are
  * serialised by a mutex.  The handle's own stream is a blocking stream, so a

@@ -30,6 +30,7 @@ using zolo::Context;
 using zolo::CudaFailure;
 
 constexpr int kCudaBase = -1000;
+constexpr int kWaitBase = -2000;  // a bounded wait inside a kernel timed out (code 9xx)
 
 // Makes the handle's device current for the call and restores the caller's current
 // device on every exit path.
@@ -53,6 +54,7 @@ int guarded(zolo_handle_t h, F&& f) {
     DeviceGuard dg(h->ctx.device());
     const int r = f(h->ctx);
     h->ctx.sync_and_free_retired();  // blocks replaced while the call ran
+    if (const int fault = h->ctx.take_fault()) return r < 0 ? r : kWaitBase - fault;
     return r;
   } catch (const CudaFailure& e) {
     return kCudaBase - static_cast<int>(e.err);

@@ -14,6 +14,21 @@ Context::Context(int device) : device_(device) {
   ck(cudaDeviceGetStreamPriorityRange(&lo, &hi));
   ck(cudaStreamCreateWithPriority(&side_, cudaStreamDefault, hi));
   for (auto& e : ev_) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  void* f = nullptr;
+  ck(cudaHostAlloc(&f, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+  fault_ = static_cast<int*>(f);  // one address for host and device (unified addressing)
+  *fault_ = 0;
+}
+
+int Context::take_fault() {
+  volatile int* f = fault_;
+  int code = *f;
+  if (code) *f = 0;
+  for (auto& w : workers) {
+    const int wc = w->take_fault();
+    if (!code) code = wc;
+  }
+  return code;
 }
 
 Context::~Context() {
@@ -22,6 +37,7 @@ Context::~Context() {
     if (e) cudaEventDestroy(e);
   if (side_) cudaStreamDestroy(side_);
   if (own_stream_) cudaStreamDestroy(own_stream_);
+  if (fault_) cudaFreeHost(fault_);
 }
 
 void Context::drop_graphs() {

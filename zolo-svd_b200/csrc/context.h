@@ -168,6 +168,11 @@ class Context {
   double* dpartial();  // 4096 doubles
   int* dinfo();        // 1024 ints
   int* oz_status_word();  // status of the INT8-emulated products (zeroed when allocated)
+  // word in mapped host memory that a kernel writes when one of its bounded waits timed out
+  int* fault_word() { return fault_; }
+  // the first fault code of this context and its workers since the last call (cleared), 0 = none;
+  // complete once the streams have been synchronized
+  int take_fault();
 
  private:
   int device_;
@@ -179,6 +184,7 @@ class Context {
   std::multimap<size_t, void*> pool_;
   std::mutex pool_mu_;
   uint64_t alloc_gen_ = 0;
+  int* fault_ = nullptr;
   void* grow(const std::string& name, size_t bytes);
 };
 

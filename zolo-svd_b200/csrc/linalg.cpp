@@ -387,7 +387,7 @@ void geqrf(Context& c, int mtot, int n, int m_top, Mat W, double* tau, double* T
       Profiler::Rec rec;
       if (c.prof.on) c.prof.begin(1, 2.0 * R.mp * static_cast<double>(jb) * jb * batch, st, &rec);
       ck(qr_panel(R.mp, jb, W.at(j, j).p, W.ld, W.stride, tau + j, n, T + pj * PW * PW, strideT, Vp.p, Vp.ld,
-                  Vp.stride, batch, st, R.split, R.gap));
+                  Vp.stride, batch, st, R.split, R.gap, c.fault_word()));
       if (c.prof.on) c.prof.end(rec, st);
       c.stats.launches++;
       const int nc = jend - j - jb;

@@ -2,8 +2,13 @@
 // [X; sqrt(c) I] (mpdgeqrf.f:252-313 / PDGEQR2 semantics, LAPACK dlarfg and
 // dlarft conventions) on one thread-block cluster per panel.
 //
-// The m x w panel (w <= 32) is split by rows over the CL CTAs of a cluster;
-// each CTA keeps its rows in shared memory when they fit.  Inside a CTA the
+// The m x w panel (w <= 32) is split by rows over the CL CTAs of a cluster.  A panel is a chain
+// of 32 dependent columns, each a reduction over all rows, so latency bounds it: up to 8192 rows
+// it stays in registers (qr_panel_reg_kernel, 1.1 us a column at m = 1024 and 2 us at m = 8192;
+// the shared-memory kernel below took 4.2 and 4.7 us).
+//
+// Larger panels run on qr_panel_kernel: each CTA keeps its rows in shared memory when they fit,
+// in global memory otherwise.  Inside a CTA the
 // work is column-parallel: thread (c, g) owns column c of the rows
 // r = g, g+8, g+16, ... of its chunk, so every phase is a short scalar loop
 // over independent rows and the row sums are 3 warp shuffles.  Column k costs
@@ -53,6 +58,7 @@ struct PanelArgs {
   int64_t strideT;
   double* V;
   int64_t ldv, strideV;
+  int* status;  // written when a wait between the CTAs timed out
 };
 
 ZDEV double group_sum8(double v) {
@@ -355,6 +361,326 @@ __global__ void __launch_bounds__(QT) qr_panel_kernel(PanelArgs p) {
   cluster.sync();  // no CTA leaves while others may still read its shared memory
 }
 
+// ---- register-resident panel ----
+// The panel of a cluster's CTA lives in registers: warp q holds 8 RN consecutive local rows;
+// thread (g = lane / 4, t = lane % 4) the rows g, g + 8, ... of them and the columns
+// 2t + (j & 1) + 8 (j >> 1), j = 0 .. 7.  Column k costs one pass over the registers, two CTA
+// barriers and one exchange between the CTAs:
+//   * x, the entries of column k below the pivot, comes from the owning lane of each quad by a
+//     shuffle; p_c = sum_r x_r a_rc for ALL 32 columns is reduced over the warp by seven
+//     shuffles (8 values over 8 lanes, halved at every stage) and over the warps by warp 0, which
+//     sends the CTA's sums into every CTA's receive slots (st.async on the receiver's mbarrier:
+//     no fence or cluster barrier on the path);
+//   * warp 0 of every CTA waits for the slots and sums them in rank order (bit-identical
+//     everywhere): p_k = ||x||^2 gives beta, tau and scal (dlarfg), p_c for c > k the update's
+//     v^T a_c = a_kc + scal p_c, and p_c for c < k the dlarft product v_c^T v_k = v_kc + scal p_c
+//     (sent to the last CTA only, whose warp 1 forms T column by column while warp 0 waits);
+//   * update a_rc += x_r (v^T a_c) / beta (tau scal = -1/beta; the pivot row is x = alpha - beta).
+// Measured per column at m = 1024 (8 CTAs of 4 warps): dots and shuffles 330 clocks, the exchange
+// 570, norm and reciprocals 330, update 280.  With cluster barriers instead of the mbarrier
+// sends the exchange took 1050, and a barrier with release semantics alone is 420.
+template <int NW>
+struct RegShared {
+  double recv[2][QCL][QW];  // sums of every CTA (by rank), double-buffered by column parity
+  double prow_in[2][QW];    // pivot row k, from the CTA holding it
+  double part[NW][QW];      // this CTA's sums by warp
+  double prow[QW];          // pivot row k if this CTA holds it
+  double w[QW];             // (v^T a_c) / beta for c > k, 0 otherwise
+  double sc[4];             // scal, beta, alpha - beta
+  double Z[2][QW];          // Z[k & 1][c] = v_c^T v_k, c < k
+  double tau[QW];
+  double T[QW][QW];         // T[j][i] = T(i, j)
+  unsigned long long bar[2];
+  uint32_t peer[QCL];  // shared-window addresses of this struct in the other CTAs, own CTA first
+  int abort;
+};
+
+ZDEV uint32_t cluster_addr(const void* p, int rank) {
+  uint32_t l = static_cast<uint32_t>(__cvta_generic_to_shared(p)), r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(l), "r"(rank));
+  return r;
+}
+// 8 bytes into another CTA's shared memory, counted by its mbarrier
+ZDEV void cluster_send(uint32_t addr, double v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(addr), "d"(v),
+               "r"(bar)
+               : "memory");
+}
+ZDEV void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+constexpr long long kPanelTimeoutCycles = 2000000000LL;  // about a second
+// Bounded wait of one warp on its CTA's mbarrier phase.
+ZDEV bool panel_wait(uint32_t bar, uint32_t parity) {
+  const long long t0 = clock64();
+  while (true) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if (clock64() - t0 > kPanelTimeoutCycles) return false;
+  }
+}
+
+// This lane's value into the same place of every CTA's struct (only the last CTA's unless `all`),
+// counted by that CTA's barrier.  Destinations are staggered by rank, so that the CTAs do not send
+// to one CTA at the same time, and their addresses come from a table: mapa per destination
+// made the 16 sends 1900 clocks, the table 400.
+template <class Sh>
+ZDEV void panel_send(Sh& S, const void* slot, const void* bar, double v, bool all, int rank, int CL) {
+  const uint32_t so = static_cast<uint32_t>(static_cast<const char*>(slot) - reinterpret_cast<const char*>(&S));
+  const uint32_t bo = static_cast<uint32_t>(static_cast<const char*>(bar) - reinterpret_cast<const char*>(&S));
+  const int ql = CL - 1 - rank;  // table index of the last CTA
+#pragma unroll
+  for (int q4 = 0; q4 < QCL; q4 += 4) {
+    if (q4 < CL) {
+      const uint4 b = *reinterpret_cast<const uint4*>(&S.peer[q4]);
+      const uint32_t base[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (q4 + u < CL && (all || q4 + u == ql)) cluster_send(base[u] + so, v, base[u] + bo);
+    }
+  }
+}
+
+// Column k of T by one warp (dlarft, forward, columnwise): T(k,k) = tau_k,
+// T(i,k) = -tau_k sum_{i <= j < k} T(i,j) v_j^T v_k; lane i forms row i.
+ZDEV void panel_t_column(double (*T)[QW], const double* z, double tau, int k) {
+  const int lane = threadIdx.x & 31;
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  int j = 0;
+  for (; j + 4 <= k; j += 4) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) s[u] = fma(T[j + u][lane], z[j + u], s[u]);
+  }
+  for (; j < k; ++j) s[0] = fma(T[j][lane], z[j], s[0]);
+  const double v = -tau * ((s[0] + s[1]) + (s[2] + s[3]));
+  T[k][lane] = lane == k ? tau : (lane < k ? v : 0.0);
+}
+
+// Factors the panel held in a[][] (local rows lr(i) = 8 RN warp + g + 8 i, global row r0 + lr; rows
+// at or past nloc hold zeros).  On return (all warps past a CTA barrier) S.tau is complete in
+// every CTA and S.T in the last one.  False after a timed-out wait.
+template <int NW, int RN>
+ZDEV bool panel_factor(double (&a)[RN][8], RegShared<NW>& S, int w, int r0, int nloc, int rank, int CL) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int rbase = r0 + warp * 8 * RN + g;  // global row of a[0]
+  // the column whose warp sum ends in this lane after the halving stages
+  const int jr = ((lane & 16) ? 4 : 0) + ((lane & 8) ? 2 : 0) + ((lane & 4) ? 1 : 0);
+  const int cr = 2 * t + (jr & 1) + 8 * (jr >> 1);
+  const bool h4 = lane & 16, h3 = lane & 8, h2 = lane & 4;
+  const bool last = rank == CL - 1;
+  const uint32_t bar0 = static_cast<uint32_t>(__cvta_generic_to_shared(&S.bar[0]));
+#pragma unroll
+  for (int grp = 0; grp < 4; ++grp) {
+#pragma unroll 1
+    for (int tt = 0; tt < 4; ++tt) {
+#pragma unroll
+      for (int par = 0; par < 2; ++par) {
+        const int k = 8 * grp + 2 * tt + par;
+        if (k >= w) goto done;
+        const int jk = 2 * grp + par;
+        constexpr int kParity[2] = {0, 1};
+        const int buf = kParity[par];
+        double x[RN];
+#pragma unroll
+        for (int i = 0; i < RN; ++i) {
+          const double v = __shfl_sync(0xffffffffu, a[i][jk], (lane & ~3) | tt);
+          x[i] = (rbase + 8 * i > k) ? v : 0.0;
+        }
+        const int kl = k - r0;
+        const bool owner = kl >= 0 && kl < nloc;
+        if (owner && kl / (8 * RN) == warp) {
+#pragma unroll
+          for (int i = 0; i < RN; ++i)
+            if (rbase + 8 * i == k) {
+#pragma unroll
+              for (int j = 0; j < 8; j += 2)
+                *reinterpret_cast<double2*>(&S.prow[2 * t + 4 * j]) = make_double2(a[i][j], a[i][j + 1]);
+            }
+        }
+        double p[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          p[j] = x[0] * a[0][j];
+#pragma unroll
+          for (int i = 1; i < RN; ++i) p[j] = fma(x[i], a[i][j], p[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const double keep = h4 ? p[j + 4] : p[j], send = h4 ? p[j] : p[j + 4];
+          p[j] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const double keep = h3 ? p[j + 2] : p[j], send = h3 ? p[j] : p[j + 2];
+          p[j] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+        }
+        {
+          const double keep = h2 ? p[1] : p[0], send = h2 ? p[0] : p[1];
+          S.part[warp][cr] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+        }
+        __syncthreads();
+        if (warp == 0) {
+          double s4[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+          for (int q = 0; q < NW; ++q) s4[q & 3] += S.part[q][lane];
+          double sum = (s4[0] + s4[1]) + (s4[2] + s4[3]), pr;
+          if (CL > 1) {
+            const uint32_t bar = bar0 + 8 * buf;
+            // columns c >= k to every CTA, c < k to the last one only; the pivot row by warp 1
+            if (lane == 0) {
+              const int bytes = (last ? QW : QW - k) * 8 * CL + QW * 8;
+              asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+                           : "memory");
+            }
+            panel_send(S, &S.recv[buf][rank][lane], &S.bar[buf], sum, lane >= k, rank, CL);
+            if (!panel_wait(bar, (k >> 1) & 1)) S.abort = 1;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) s4[q] = 0.0;
+#pragma unroll
+            for (int q = 0; q < QCL; ++q)
+              if (q < CL) s4[q & 3] += S.recv[buf][q][lane];
+            sum = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+            pr = S.prow_in[buf][lane];
+          } else {
+            pr = S.prow[lane];
+          }
+          const double s0 = __shfl_sync(0xffffffffu, sum, k);
+          const double alpha = __shfl_sync(0xffffffffu, pr, k);
+          double beta = alpha, tau = 0.0, scal = 0.0, rb = 0.0;
+          if (s0 != 0.0) {
+            // norm and its reciprocal from one rsqrt (norm corrected by a Newton step)
+            const double n2 = fma(alpha, alpha, s0), r = rsqrt(n2);
+            double nrm = n2 * r;
+            nrm = fma(0.5 * r, fma(-nrm, nrm, n2), nrm);
+            beta = -copysign(nrm, alpha);
+            rb = -copysign(r, alpha);
+            scal = 1.0 / (alpha - beta);
+            tau = (beta - alpha) * rb;
+          }
+          const double vta = fma(scal, sum, pr);
+          S.w[lane] = lane > k ? vta * rb : 0.0;
+          S.Z[buf][lane] = vta;
+          if (lane == 0) {
+            S.sc[0] = scal;
+            S.sc[1] = beta;
+            S.sc[2] = alpha - beta;
+            S.tau[k] = tau;
+          }
+        } else if (warp == 1) {
+          if (CL > 1 && owner) {
+            const double pr = S.prow[lane];
+            panel_send(S, &S.prow_in[buf][lane], &S.bar[buf], pr, true, rank, CL);
+          }
+          // the previous column of T, while warp 0 waits
+          if (last && k > 0) panel_t_column(S.T, S.Z[buf ^ 1], S.tau[k - 1], k - 1);
+        }
+        __syncthreads();
+        if (CL > 1 && S.abort) return false;
+        const double scal = S.sc[0], beta = S.sc[1], xp = S.sc[2];
+        double xu[RN];
+#pragma unroll
+        for (int i = 0; i < RN; ++i) xu[i] = (rbase + 8 * i == k) ? xp : x[i];
+#pragma unroll
+        for (int j = 2 * grp; j < 8; j += 2) {
+          const double2 wj = *reinterpret_cast<const double2*>(&S.w[2 * t + 4 * j]);
+#pragma unroll
+          for (int i = 0; i < RN; ++i) {
+            a[i][j] = fma(xu[i], wj.x, a[i][j]);
+            a[i][j + 1] = fma(xu[i], wj.y, a[i][j + 1]);
+          }
+        }
+        if (t == tt) {
+#pragma unroll
+          for (int i = 0; i < RN; ++i) {
+            if (rbase + 8 * i > k) a[i][jk] = x[i] * scal;
+            else if (rbase + 8 * i == k) a[i][jk] = beta;
+          }
+        }
+      }
+    }
+  }
+done:
+  if (last && warp == 1) panel_t_column(S.T, S.Z[(w - 1) & 1], S.tau[w - 1], w - 1);
+  return true;
+}
+
+template <int NW, int RN>
+__global__ void __launch_bounds__(NW * 32, 1) qr_panel_reg_kernel(PanelArgs p) {
+  __shared__ __align__(16) RegShared<NW> S;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = static_cast<int>(cluster.block_rank());
+  const int CL = static_cast<int>(cluster.num_blocks());
+  const int b = blockIdx.y, m = p.m, w = p.w;
+  const int r0 = rank * p.rows_per;
+  const int nloc = max(min(m, r0 + p.rows_per) - r0, 0);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int l0 = warp * 8 * RN + g;
+  const int64_t lda = p.lda;
+  // element offsets of this thread's rows (past the row gap) and first column
+  double* A = p.A + b * p.strideA + r0 + l0 + 2 * t * lda;
+  int64_t ro[RN];
+#pragma unroll
+  for (int i = 0; i < RN; ++i) ro[i] = 8 * i + (r0 + l0 + 8 * i >= p.split ? p.gap : 0);
+  double a[RN][8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const bool in = 2 * t + (j & 1) + 8 * (j >> 1) < w;
+    const double* col = A + ((j & 1) + 8 * (j >> 1)) * lda;
+#pragma unroll
+    for (int i = 0; i < RN; ++i) a[i][j] = (in && l0 + 8 * i < nloc) ? col[ro[i]] : 0.0;
+  }
+  if (CL > 1) {
+    if (threadIdx.x == 0) {
+      S.abort = 0;
+      for (int q = 0; q < CL; ++q) S.peer[q] = cluster_addr(&S, (rank + q) & (CL - 1));
+      for (int q = 0; q < 2; ++q)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(
+                         static_cast<uint32_t>(__cvta_generic_to_shared(&S.bar[q])))
+                     : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // every CTA of the cluster runs, its barriers ready, before the first send to it
+    cluster_sync_all();
+  }
+  if (!panel_factor<NW, RN>(a, S, w, r0, nloc, rank, CL)) {
+    if (threadIdx.x == 0 && p.status) {
+      *static_cast<volatile int*>(p.status) = 911;
+      __threadfence_system();
+    }
+    cluster_sync_all();  // no CTA leaves while others may still send to it
+    return;
+  }
+  double* V = p.V + b * p.strideV + r0 + l0 + 2 * t * p.ldv;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int c = 2 * t + (j & 1) + 8 * (j >> 1);
+    if (c >= w) continue;
+    double* col = A + ((j & 1) + 8 * (j >> 1)) * lda;
+    double* vcol = V + ((j & 1) + 8 * (j >> 1)) * p.ldv;
+#pragma unroll
+    for (int i = 0; i < RN; ++i) {
+      if (l0 + 8 * i >= nloc) continue;
+      const int r = r0 + l0 + 8 * i;
+      col[ro[i]] = a[i][j];
+      vcol[8 * i] = r > c ? a[i][j] : (r == c ? 1.0 : 0.0);
+    }
+  }
+  if (rank == CL - 1 && warp == 1) {
+    __syncwarp();
+    double* T = p.T + b * p.strideT;
+#pragma unroll 4
+    for (int j = 0; j < QW; ++j) T[lane + j * QW] = j < w ? S.T[j][lane] : 0.0;
+    if (lane < w) p.tau[b * p.strideTau + lane] = S.tau[lane];
+  }
+}
+
 __global__ void extract_v_kernel(int m, int w, const double* __restrict__ A, int64_t lda, int64_t strideA,
                                  double* V, int64_t ldv, int64_t strideV, int split, int64_t gap) {
   const double* Ab = A + blockIdx.y * strideA;
@@ -445,6 +771,27 @@ cudaError_t launch_panel(const PanelArgs& pa, int cl, int batch, size_t smem, cu
   return cudaLaunchKernelEx(&cfg, qr_panel_kernel<SMEM>, pa);
 }
 
+template <int NW, int RN>
+cudaError_t launch_reg(const PanelArgs& pa, int cl, int batch, cudaStream_t st) {
+  static std::atomic<int> attr_set[kMaxDevices];
+  const cudaError_t e = once_per_device(attr_set, [] {
+    return cudaFuncSetAttribute(qr_panel_reg_kernel<NW, RN>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  });
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cl, batch, 1);
+  cfg.blockDim = dim3(NW * 32, 1, 1);
+  cfg.stream = st;
+  cudaLaunchAttribute attr_l[1];
+  attr_l[0].id = cudaLaunchAttributeClusterDimension;
+  attr_l[0].val.clusterDim.x = cl;
+  attr_l[0].val.clusterDim.y = 1;
+  attr_l[0].val.clusterDim.z = 1;
+  cfg.attrs = attr_l;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, qr_panel_reg_kernel<NW, RN>, pa);
+}
+
 // 16-CTA clusters are non-portable: use them only if the device can place one
 // with the largest shared-memory footprint; otherwise the portable 8.
 int max_cluster() {
@@ -471,11 +818,39 @@ int max_cluster() {
   });
 }
 
+// Cluster size and warps per CTA (32 rows each) of the register-resident panel; false when the
+// rows do not fit (m > 8192 with clusters of 16).  The cheapest configuration by the measured
+// times of one 32-column panel alone on the GPU: a CTA of 4 / 8 / 16 warps 26 / 30 / 45 us, and
+// the exchange 7 us more with clusters of 2 or 4, 10 us with 8, 16.5 us with 16 (m = 512: 33 us on
+// 4 CTAs of 4 warps against 47 us on one of 16; m = 8192: 63 us on 16 x 16).  A batch that does
+// not fit the GPU at once pays per wave: its members then take fewer, larger CTAs.
+bool reg_config(int m, int batch, int maxcl, int* cl, int* nw) {
+  double best = 1e300;
+  for (int n : {4, 8, 16}) {
+    const double t_cta = n == 4 ? 26.0 : (n == 8 ? 30.0 : 45.0);
+    const int per_sm = n == 4 ? 2 : 1;
+    for (int c = 1; c <= maxcl; c *= 2) {
+      if (static_cast<int64_t>(c) * n * 32 < m) continue;
+      const double t = t_cta + (c == 1 ? 0.0 : (c <= 4 ? 7.0 : (c == 8 ? 10.0 : 16.5)));
+      const double waves = static_cast<double>(c) * batch / (static_cast<double>(num_sms()) * per_sm);
+      const double cost = t * std::max(1.0, waves);
+      if (cost < best) {
+        best = cost;
+        *cl = c;
+        *nw = n;
+      }
+    }
+  }
+  return best < 1e300;
+}
+
 }  // namespace
 
 int qr_panel_config(int m, int w) {
   const int maxcl = max_cluster();
-  int cl = 1;
+  int cl = 1, nw = 0;
+  if (reg_config(m, 1, maxcl, &cl, &nw)) return cl;
+  cl = 1;
   while (cl < maxcl && (static_cast<size_t>(((m + cl - 1) / cl + 7) / 16 * 16 + 8) * w * 8 > SMEM_CHUNK_CAP ||
                         (m + cl - 1) / cl > 512))
     cl *= 2;
@@ -485,7 +860,7 @@ int qr_panel_config(int m, int w) {
 
 cudaError_t qr_panel(int m, int w, double* A, int64_t lda, int64_t strideA, double* tau, int64_t strideTau,
                      double* T, int64_t strideT, double* Vexp, int64_t ldv, int64_t strideV, int batch,
-                     cudaStream_t st, int split, int64_t gap) {
+                     cudaStream_t st, int split, int64_t gap, int* status) {
   if (m <= 0 || w <= 0 || batch <= 0) return cudaSuccess;
   if (w > QW || m < w || gap < 0 || (gap > 0 && split < w)) return cudaErrorInvalidValue;
   const int maxcl = max_cluster();
@@ -511,6 +886,16 @@ cudaError_t qr_panel(int m, int w, double* A, int64_t lda, int64_t strideA, doub
   pa.V = Vexp;
   pa.ldv = ldv;
   pa.strideV = strideV;
+  pa.status = status;
+  int rcl = 0, rnw = 0;
+  if (reg_config(m, batch, maxcl, &rcl, &rnw)) {
+    pa.rows_per = (m + rcl - 1) / rcl;
+    switch (rnw) {
+      case 4: return launch_reg<4, 4>(pa, rcl, batch, st);
+      case 8: return launch_reg<8, 4>(pa, rcl, batch, st);
+      default: return launch_reg<16, 4>(pa, rcl, batch, st);
+    }
+  }
   const size_t chunk = static_cast<size_t>(pa.rp_ld) * w * 8;
   if (chunk <= SMEM_CHUNK_CAP) return launch_panel<true>(pa, cl, batch, shared_base() + chunk, st);
   return launch_panel<false>(pa, cl, batch, shared_base(), st);
