@@ -561,7 +561,10 @@ ZDEV bool panel_factor(double (&a)[RN][8], RegShared<NW>& S, int w, int r0, int 
             nrm = fma(0.5 * r, fma(-nrm, nrm, n2), nrm);
             beta = -copysign(nrm, alpha);
             rb = -copysign(r, alpha);
-            scal = 1.0 / (alpha - beta);
+            // 1/(alpha - beta), its magnitude |alpha| + norm >= norm, as rsqrt of its square: a division's
+            // chain is 150 clocks longer
+            const double z = alpha - beta;
+            scal = copysign(rsqrt(z * z), z);
             tau = (beta - alpha) * rb;
           }
           const double vta = fma(scal, sum, pr);
