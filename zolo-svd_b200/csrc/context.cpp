@@ -112,10 +112,6 @@ void Context::release_all() {
     pool_.clear();
   }
   ++alloc_gen_;
-  if (splitk_.ptr) cudaFree(splitk_.ptr);
-  if (splitk_side_.ptr) cudaFree(splitk_side_.ptr);
-  splitk_ = Scratch{};
-  splitk_side_ = Scratch{};
 }
 
 void* Context::grow(const std::string& name, size_t bytes) {
@@ -144,22 +140,6 @@ double* Context::buf(const std::string& name, size_t elems) {
 
 int* Context::ibuf(const std::string& name, size_t elems) {
   return static_cast<int*>(grow(name, elems * sizeof(int)));
-}
-
-void Context::ensure_splitk(size_t bytes, bool side) {
-  Scratch& s = side ? splitk_side_ : splitk_;
-  if (s.bytes >= bytes) return;
-  if (s.ptr) {
-    retired_.push_back(s.ptr);  // freed by free_retired, as in grow
-    ++alloc_gen_;
-    ++reallocs;
-  }
-  s.ptr = nullptr;
-  s.bytes = 0;
-  void* p = nullptr;
-  ck(cudaMalloc(&p, bytes));
-  s.ptr = static_cast<double*>(p);
-  s.bytes = bytes;
 }
 
 cudaEvent_t Profiler::take() {

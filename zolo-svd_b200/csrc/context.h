@@ -88,9 +88,6 @@ class Context {
   // Named cached device buffer of at least `elems` doubles (grow-only).
   double* buf(const std::string& name, size_t elems);
   int* ibuf(const std::string& name, size_t elems);
-  // split-K partial sums; GEMMs on the side stream have their own
-  Scratch& splitk(bool side = false) { return side ? splitk_side_ : splitk_; }
-  void ensure_splitk(size_t bytes, bool side = false);
   void release_all();
 
   Stats stats;
@@ -179,7 +176,6 @@ class Context {
   cudaStream_t stream_ = nullptr, own_stream_ = nullptr, side_ = nullptr;
   cudaEvent_t ev_[4] = {nullptr, nullptr, nullptr, nullptr};
   std::map<std::string, std::pair<void*, size_t>> bufs_;
-  Scratch splitk_, splitk_side_;
   std::vector<void*> retired_;
   std::multimap<size_t, void*> pool_;
   std::mutex pool_mu_;

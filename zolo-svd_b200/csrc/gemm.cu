@@ -7,7 +7,9 @@
 // TF/s on a 4096^3 main-loop probe against 30.3 for 128x128 tiles with one CTA
 // per SM; the FP64 tensor pipe saturates at 37.0).  Padded shared-memory
 // layouts make every fragment load a conflict-free LDS.128 (or LDS.64 for
-// op(B)=B^T).
+// op(B)=B^T).  Products too small for that grid take 32x32 tiles with four warps, and a long K
+// is split over the CTAs of a cluster, which reduce through distributed shared memory
+// (1024 x 512 x 512: 72 -> 30 us against one launch with scratch in global memory).
 //
 // Index permutations (free because they are applied consistently):
 //   * inside each 16-row MMA tile, logical row g <-> physical row 2g and
@@ -18,13 +20,17 @@
 #include "common.cuh"
 #include "kernels.h"
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
+
+namespace cg = cooperative_groups;
 
 namespace zolo {
 
 namespace {
 
-constexpr int BK = 16, NT = 256;
+constexpr int BK = 16;
 constexpr int LDA_T = BK + 4;  // sA[m][k]  (op(A) = A^T)
 constexpr int LDB_N = BK + 8;  // sB[n][k]  (op(B) = B)
 
@@ -32,30 +38,30 @@ constexpr int LDB_N = BK + 8;  // sB[n][k]  (op(B) = B)
 template <int BM_, int BN_, int WM_, int WN_, int ST_ = 4, int MINB_ = 1>
 struct Cfg {
   static constexpr int BM = BM_, BN = BN_, WM = WM_, WN = WN_, STAGES = ST_, MINB = MINB_;
+  static constexpr int NT = WM * WN * 32;
   static constexpr int MI = BM / WM / 16, NJ = BN / WN / 8;
   static constexpr int LDA_N = BM + 2;  // sA[k][m]  (op(A) = A)
   static constexpr int LDB_T = BN + 2;  // sB[k][n]  (op(B) = B^T)
-  static_assert(WM * WN * 32 == NT, "8 warps");
   __host__ __device__ static constexpr int a_elems(bool ta) { return ta ? BM * LDA_T : BK * LDA_N; }
   __host__ __device__ static constexpr int b_elems(bool tb) { return tb ? BK * LDB_T : BN * LDB_N; }
-  static constexpr int smem(bool ta, bool tb) { return ST_ * (a_elems(ta) + b_elems(tb)) * 8; }
+  __host__ __device__ static constexpr int smem(bool ta, bool tb) { return ST_ * (a_elems(ta) + b_elems(tb)) * 8; }
 };
 using CfgWide = Cfg<64, 128, 2, 4, 3, 2>;     // general: 2 CTAs / SM, warp tile 32x32
 using CfgSkinnyM = Cfg<32, 64, 1, 8, 4, 3>;    // M <= 32 (V^T W products of the QR updates)
 using CfgSmall = Cfg<64, 64, 2, 4, 2, 3>;      // K <= 64 rank-k updates and N <= 64: 3 CTAs / SM
 using CfgTri = Cfg<64, 64, 2, 4, 3, 3>;        // lower-triangle output (square tiles): 3 CTAs / SM
+using CfgTiny = Cfg<32, 32, 2, 2, 4, 4>;       // products too small to fill the GPU with larger tiles
 
 struct KParams {
   GemmArgs g;
   int tiles_m, tiles_n;
   int splitk;
   int preload;  // C loaded into the accumulators up front (rank-k updates)
-  double* P;  // split-K partials
-  int64_t ldp;
 };
 
 template <class C, bool TA, bool TB, bool V16>
-__global__ void __launch_bounds__(NT, C::MINB) dgemm_kernel(KParams kp) {
+__global__ void __launch_bounds__(C::NT, C::MINB) dgemm_kernel(KParams kp) {
+  constexpr int NT = C::NT;
   constexpr int BM = C::BM, BN = C::BN, MI = C::MI, NJ = C::NJ;
   constexpr int LDA_N = C::LDA_N, LDB_T = C::LDB_T;
   constexpr int AE = C::a_elems(TA), BE = C::b_elems(TB);
@@ -252,22 +258,44 @@ __global__ void __launch_bounds__(NT, C::MINB) dgemm_kernel(KParams kp) {
 
   // ---- epilogue ----
   if (kp.splitk > 1) {
-    double* P = kp.P + (static_cast<int64_t>(split) * p.batch + bz) * kp.ldp * N;
+    // the slices of a tile are one cluster: every CTA leaves its partial tile in shared memory,
+    // and each then sums its share of the columns over the cluster in slice order and writes it
+    // (a pass through global scratch cost a second launch, 2.5 us and its gap)
+    constexpr int LDP = BM + 2;
+    static_assert(BN * LDP * 8 <= C::smem(TA, TB), "partial tile fits the pipeline's buffers");
+    cg::cluster_group cluster = cg::this_cluster();
+    __syncthreads();
+    double* P = smem;
 #pragma unroll
     for (int i = 0; i < MI; ++i)
 #pragma unroll
       for (int j = 0; j < NJ; ++j) {
-        const int r = m0 + wm + i * 16 + 2 * g;
-        const int c = n0 + wn + j * 8 + 2 * t;
+        const int r = wm + i * 16 + 2 * g, c = wn + j * 8 + 2 * t;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int cc = c + h;
-          if (cc >= N) continue;
-          double* dst = P + r + static_cast<int64_t>(cc) * kp.ldp;
-          if (r < M) dst[0] = acc[i][j][h];
-          if (r + 1 < M) dst[1] = acc[i][j][2 + h];
-        }
+        for (int h = 0; h < 2; ++h)
+          *reinterpret_cast<double2*>(P + r + (c + h) * LDP) = make_double2(acc[i][j][h], acc[i][j][2 + h]);
       }
+    cluster.sync();
+    const double al = p.alpha * (p.alpha_vec ? p.alpha_vec[bz] : 1.0);
+    double* Cb = p.C + static_cast<int64_t>(bz) * p.strideC;
+    const int S = kp.splitk, per = (BN + S - 1) / S;
+    const int c0 = split * per, c1 = min(BN, c0 + per);
+    for (int e = tid; e < (c1 - c0) * (BM / 2); e += NT) {
+      const int r = (e % (BM / 2)) * 2, c = c0 + e / (BM / 2);
+      double s0 = 0.0, s1 = 0.0;
+#pragma unroll 4
+      for (int q = 0; q < S; ++q) {
+        const double2 v = *reinterpret_cast<const double2*>(cluster.map_shared_rank(P, q) + r + c * LDP);
+        s0 += v.x;
+        s1 += v.y;
+      }
+      const int gr = m0 + r, gc = n0 + c;
+      if (gc >= N) continue;
+      double* dst = Cb + gr + static_cast<int64_t>(gc) * p.ldc;
+      if (gr < M && (!p.tri || gr >= gc)) dst[0] = p.beta != 0.0 ? fma(p.beta, dst[0], al * s0) : al * s0;
+      if (gr + 1 < M && (!p.tri || gr + 1 >= gc)) dst[1] = p.beta != 0.0 ? fma(p.beta, dst[1], al * s1) : al * s1;
+    }
+    cluster.sync();  // no CTA leaves while others read its partial tile
     return;
   }
   double* C_ = p.C + static_cast<int64_t>(bz) * p.strideC;
@@ -304,26 +332,6 @@ __global__ void __launch_bounds__(NT, C::MINB) dgemm_kernel(KParams kp) {
     }
 }
 
-__global__ void splitk_reduce_kernel(GemmArgs p, int splitk, const double* P, int64_t ldp) {
-  const int64_t total = static_cast<int64_t>(p.M) * p.N;
-  const int bz = blockIdx.y;
-  const double alpha = p.alpha * (p.alpha_vec ? p.alpha_vec[bz] : 1.0);
-  double* C = p.C + static_cast<int64_t>(bz) * p.strideC;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % p.M);
-    const int j = static_cast<int>(e / p.M);
-    if (p.tri && i < j) continue;
-    double s = 0.0;
-    for (int q = 0; q < splitk; ++q)
-      s += P[(static_cast<int64_t>(q) * p.batch + bz) * ldp * p.N + i + static_cast<int64_t>(j) * ldp];
-    double* dst = C + i + static_cast<int64_t>(j) * p.ldc;
-    double v = alpha * s;
-    if (p.beta != 0.0) v += p.beta * *dst;
-    *dst = v;
-  }
-}
-
 template <class C, bool TA, bool TB, bool V16>
 cudaError_t launch_t(const KParams& kp, dim3 grid, cudaStream_t st) {
   static std::atomic<int> attr_set[kMaxDevices];
@@ -332,8 +340,23 @@ cudaError_t launch_t(const KParams& kp, dim3 grid, cudaStream_t st) {
                                 C::smem(TA, TB));
   });
   if (attr != cudaSuccess) return attr;
-  dgemm_kernel<C, TA, TB, V16><<<grid, NT, C::smem(TA, TB), st>>>(kp);
-  return cudaGetLastError();
+  if (kp.splitk <= 1) {
+    dgemm_kernel<C, TA, TB, V16><<<grid, C::NT, C::smem(TA, TB), st>>>(kp);
+    return cudaGetLastError();
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(C::NT, 1, 1);
+  cfg.dynamicSmemBytes = C::smem(TA, TB);
+  cfg.stream = st;
+  cudaLaunchAttribute la[1];
+  la[0].id = cudaLaunchAttributeClusterDimension;
+  la[0].val.clusterDim.x = 1;
+  la[0].val.clusterDim.y = kp.splitk;
+  la[0].val.clusterDim.z = 1;
+  cfg.attrs = la;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, dgemm_kernel<C, TA, TB, V16>, kp);
 }
 
 template <class C, bool V16>
@@ -351,8 +374,17 @@ cudaError_t launch_c(const KParams& kp, dim3 grid, bool v16, cudaStream_t st) {
 }
 
 // tile shape: 0 = 64x128 (general), 1 = 32x64 (M <= 32), 2 = 64x64 (K <= 64 or N <= 64),
-// 3 = 64x64 with 3 stages (lower-triangle output)
+// 3 = 64x64 with 3 stages (lower-triangle output), 4 = 32x32 (too small to fill the GPU)
 int pick_cfg(const GemmArgs& a) {
+  // Products that leave SMs idle with 64 x 64 tiles (FP64 DMMA runs at 64 FMA a clock and SM, so a
+  // tile of K = 64 alone takes 2.1 us): 32 x 32 tiles spread them wider.  Measured 64 x 64 against
+  // 32 x 32: 64^3 5.8 / 3.7 us, 1024 x 128 x 128 11.3 / 7.1, 128 x 896 x 1024 (split K) 18.3 / 15.7; past
+  // about 1.4e8 multiplications or one tile per SM the larger tiles' reuse wins
+  // (1024 x 512 x 512 30 / 44 us, 1024 x 896 x 128 17.3 / 18.5).
+  const int64_t t64 = (a.M + 63) / 64, u64 = (a.N + 63) / 64;
+  const int64_t tiles64 = (a.tri ? t64 * (t64 + 1) / 2 : t64 * u64) * a.batch;
+  const double work = static_cast<double>(a.M) * a.N * a.K * a.batch * (a.tri ? 0.5 : 1.0);
+  if (tiles64 < num_sms() && work <= 1.4e8) return 4;
   if (a.tri) return 3;
   if (a.M <= 32) return 1;
   if (a.K <= 64 || a.N <= 64) return 2;
@@ -364,7 +396,11 @@ int pick_cfg(const GemmArgs& a) {
 }
 
 void tile_dims(int cfg, int* bm, int* bn, int* per_sm) {
-  if (cfg == 1) {
+  if (cfg == 4) {
+    *bm = CfgTiny::BM;
+    *bn = CfgTiny::BN;
+    *per_sm = CfgTiny::MINB;
+  } else if (cfg == 1) {
     *bm = CfgSkinnyM::BM;
     *bn = CfgSkinnyM::BN;
     *per_sm = CfgSkinnyM::MINB;
@@ -383,19 +419,21 @@ void tile_dims(int cfg, int* bm, int* bn, int* per_sm) {
   }
 }
 
-// Split K only when the tile grid cannot fill the GPU; pick the split that fills whole
-// waves (sms * resident CTAs per SM) best, with at least 8 K tiles per split.
+// Split K only when the tile grid cannot fill the GPU; pick the split (the CTAs of one portable
+// cluster, 8 at most) that fills whole waves (sms * resident CTAs per SM) best, with at least 8
+// K tiles per split (4 of the 32 x 32 tiles).
 int choose_splitk(const GemmArgs& a, int sms) {
   if (a.splitk >= 1) return a.splitk;
   int BM, BN, per_sm;
-  tile_dims(pick_cfg(a), &BM, &BN, &per_sm);
+  const int cfg = pick_cfg(a);
+  tile_dims(cfg, &BM, &BN, &per_sm);
   const int tm = (a.M + BM - 1) / BM, tn = (a.N + BN - 1) / BN;
   const int64_t tiles = a.tri ? static_cast<int64_t>(tm) * (tm + 1) / 2 : static_cast<int64_t>(tm) * tn;
   const int64_t ctas = tiles * a.batch;
   const int64_t wave = static_cast<int64_t>(sms) * per_sm;
   if (ctas >= wave) return 1;
   const int kt = (a.K + BK - 1) / BK;
-  const int smax = std::min(32, kt / 8);
+  const int smax = std::min(8, kt / (cfg == 4 ? 4 : 8));
   if (smax < 2) return 1;
   int best = 1;
   double best_eff = static_cast<double>(ctas) / wave;  // fraction of one wave used unsplit
@@ -425,14 +463,7 @@ int num_sms() {
   });
 }
 
-size_t dgemm_splitk_bytes(const GemmArgs& a, int sms) {
-  const int s = choose_splitk(a, sms);
-  if (s <= 1) return 0;
-  const int64_t ldp = (a.M + 1) / 2 * 2;
-  return static_cast<size_t>(s) * a.batch * ldp * a.N * sizeof(double);
-}
-
-cudaError_t dgemm(GemmArgs a, const Scratch& ws, cudaStream_t st) {
+cudaError_t dgemm(GemmArgs a, cudaStream_t st) {
   if (a.M <= 0 || a.N <= 0 || a.batch <= 0) return cudaSuccess;
   if (a.tri && a.M != a.N) return cudaErrorInvalidValue;
   // 16-byte cp.async path when every tile chunk is 16-byte aligned, else 8-byte copies
@@ -457,16 +488,6 @@ cudaError_t dgemm(GemmArgs a, const Scratch& ws, cudaStream_t st) {
   kp.tiles_m = (a.M + BM - 1) / BM;
   kp.tiles_n = (a.N + BN - 1) / BN;
   kp.splitk = choose_splitk(a, sms);
-  kp.ldp = (a.M + 1) / 2 * 2;
-  kp.P = nullptr;
-  if (kp.splitk > 1) {
-    const size_t need = static_cast<size_t>(kp.splitk) * a.batch * kp.ldp * a.N * sizeof(double);
-    if (ws.ptr == nullptr || ws.bytes < need) {
-      kp.splitk = 1;  // not enough scratch: run unsplit
-    } else {
-      kp.P = ws.ptr;
-    }
-  }
   kp.preload = (kp.splitk <= 1 && a.beta != 0.0 && !a.tri && !a.kto_m && !a.alpha_vec &&
                  (a.alpha == 1.0 || a.alpha == -1.0) && (a.K <= 64 || (cfg == 2 && a.K <= 256)))
                    ? 1
@@ -478,12 +499,9 @@ cudaError_t dgemm(GemmArgs a, const Scratch& ws, cudaStream_t st) {
   const cudaError_t e = cfg == 1   ? launch_c<CfgSkinnyM>(kp, grid, v16, st)
                         : cfg == 2 ? launch_c<CfgSmall>(kp, grid, v16, st)
                         : cfg == 3 ? launch_c<CfgTri>(kp, grid, v16, st)
+                        : cfg == 4 ? launch_c<CfgTiny>(kp, grid, v16, st)
                                    : launch_c<CfgWide>(kp, grid, v16, st);
-  if (e != cudaSuccess || kp.splitk <= 1) return e;
-  const int64_t total = static_cast<int64_t>(a.M) * a.N;
-  int blocks = static_cast<int>(std::min<int64_t>((total + 255) / 256, 4 * sms));
-  splitk_reduce_kernel<<<dim3(blocks, a.batch), 256, 0, st>>>(a, kp.splitk, kp.P, kp.ldp);
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace zolo

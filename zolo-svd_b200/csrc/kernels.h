@@ -29,14 +29,7 @@ struct GemmArgs {
   int splitk = 0;   // 0 = choose; 1 = off; >1 = number of K slices
 };
 
-// Scratch for split-K partial sums (owned by the caller's context).
-struct Scratch {
-  double* ptr = nullptr;
-  size_t bytes = 0;
-};
-
-cudaError_t dgemm(GemmArgs a, const Scratch& ws, cudaStream_t st);
-size_t dgemm_splitk_bytes(const GemmArgs& a, int num_sms);
+cudaError_t dgemm(GemmArgs a, cudaStream_t st);
 // Streaming rank-k update C = beta*C + alpha*A*B (no transposes, K <= 32; update.cu).
 // dgemm dispatches to it when rank_update_applies(a).
 bool rank_update_applies(const GemmArgs& a);

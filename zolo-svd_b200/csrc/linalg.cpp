@@ -98,19 +98,16 @@ void gemm(Context& c, int transA, int transB, int M, int N, int K, double alpha,
   a.tri = tri;
   a.kfrom_n = kfrom_n;
   a.kto_m = kto_m;
-  const size_t need = dgemm_splitk_bytes(a, num_sms());
   cudaStream_t s = st ? st : c.stream();
-  const bool side = s == c.side_stream() && s != c.stream();
-  if (need) c.ensure_splitk(need, side);
   Profiler::Rec rec;
   const int cls = tri ? 6 : (M <= 32 ? 3 : (N <= 64 ? 4 : (K <= 64 ? 5 : (K <= 256 ? 8 : 0))));
   if (c.prof.on) {
     const double f = algo_flops(M, N, K, tri, kfrom_n, kto_m);
     c.prof.begin(cls, f * batch, s, &rec);
   }
-  ck(dgemm(a, c.splitk(side), s));
+  ck(dgemm(a, s));
   if (c.prof.on) c.prof.end(rec, s);
-  c.stats.launches += need ? 2 : 1;
+  c.stats.launches++;
 }
 
 void ozgemm(Context& c, int transA, int transB, int M, int N, int K, double alpha, Mat A, Mat B, double beta, Mat C,

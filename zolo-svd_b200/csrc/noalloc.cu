@@ -91,7 +91,7 @@ cudaError_t gemm_nosplit(int ta, int tb, int M, int N, int K, double alpha, cons
   g.beta = beta;
   g.tri = tri;
   g.splitk = 1;
-  return dgemm(g, Scratch{}, st);
+  return dgemm(g, st);
 }
 
 // Y = X L^{-T}; the inverse of L's diagonal block k is at dinv + (k0 + k) * 4096
