@@ -124,7 +124,7 @@ cudaError_t trtri_blocks(int n, const double* L, int64_t ldl, int64_t strideL, d
 // diagonal (unit diagonal implied), R on/above it, tau[w], T (w x w upper, ld 32)
 // of the compact WY form I - V T V^T.  Vexp receives V explicitly (m x w, ldv).
 // Row gap: with split > 0, logical row r >= split of the panel is the physical
-// row r + gap of A (two row segments; Vexp stays in logical rows).
+// row r + gap of A (two row segments; Vexp stays in logical rows).  Vexp may be null up to 8192 rows.
 cudaError_t qr_panel(int m, int w, double* A, int64_t lda, int64_t strideA, double* tau,
                      int64_t strideTau, double* T, int64_t strideT, double* Vexp, int64_t ldv,
                      int64_t strideV, int batch, cudaStream_t st, int split = 0, int64_t gap = 0,
@@ -143,6 +143,16 @@ cudaError_t block_t_init(int jb, const double* T, int64_t strideT, double* TB, i
 // P'(b) = T(b)^T * P(b) (trans=1) or T(b) * P(b) (trans=0); T w x w upper (ld 32), P w x n.
 cudaError_t apply_t(int w, int n, const double* T, int64_t strideT, double* P, int64_t ldp,
                     int64_t strideP, int trans, int batch, cudaStream_t st);
+
+// C(b) <- (I - V op(T) V^T) C(b) (reflect.cu): V(b) the m x w (w <= 32) panel that qr_panel left in
+// place (R and what is above V's unit diagonal are not read as V), T w x w upper (ld 32), op(T) = T^T
+// with `trans`, C m x nc.  V and C share the row gap (as in qr_panel).  reflect_applies: m fits.
+bool reflect_applies(int m);
+// Largest cluster the panel kernels use on the current device (16, or the portable 8).
+int panel_cluster_max();
+cudaError_t reflect(int m, int nc, int w, const double* V, int64_t ldv, int64_t strideV, const double* T,
+                    int64_t strideT, int trans, double* C, int64_t ldc, int64_t strideC, int batch, cudaStream_t st,
+                    int split = 0, int64_t gap = 0);
 
 // ---- eigen stage (jacobi.cu, elementwise.cu) ----
 struct JacobiLeaf {

@@ -359,6 +359,74 @@ static void block_t(Context& c, int jb, Mat VB, int mp, const double* T, int64_t
   }
 }
 
+// C <- (I - V op(T) V^T) C over the panel's rows, V the panel at Vp in the factored matrix and C the
+// columns at Cp (both at the panel's first row), one launch.
+static void apply_panel(Context& c, const PanelRows& R, int jb, int ncols, Mat Vp, const double* T, int64_t strideT,
+                        int trans, Mat Cp, int batch, cudaStream_t st) {
+  Profiler::Rec rec;
+  if (c.prof.on) c.prof.begin(5, 4.0 * R.mp * static_cast<double>(ncols) * jb * batch, st, &rec);
+  ck(reflect(R.mp, ncols, jb, Vp.p, Vp.ld, Vp.stride, T, strideT, trans, Cp.p, Cp.ld, Cp.stride, batch, st, R.split,
+             R.gap));
+  if (c.prof.on) c.prof.end(rec, st);
+  c.stats.launches++;
+}
+
+// Factorizations that apply every panel to all remaining columns at once (apply_panel) instead of
+// in 128-column blocks: while the trailing update fits beside the next panel the blocks' T factors
+// and products only lengthen the chain.  Measured, panelwise against blocks: QR of 1024 x 1024
+// 1.6 / 2.0 ms, 2048 x 2048 4.0 / 4.7, 4096 x 2048 8.2 / 6.3; forming Q, where nothing hides the
+// update, 1024 x 1024 0.48 / 0.63 ms, 2048 x 1024 0.93 / 0.80.
+static bool panelwise(int mtot, int n, int batch, bool qr) {
+  return reflect_applies(mtot) && static_cast<double>(mtot) * n * batch <= (qr ? 4.5e6 : 1.5e6);
+}
+
+static void factor_panel(Context& c, int mtot, int n, int m_top, bool top_tri, int j, Mat W, double* tau, double* T,
+                         int64_t strideT, Mat Vp, int batch, cudaStream_t st) {
+  const int jb = std::min(PW, n - j);
+  const PanelRows R = panel_rows(mtot, m_top, top_tri, j, jb);
+  Profiler::Rec rec;
+  if (c.prof.on) c.prof.begin(1, 2.0 * R.mp * static_cast<double>(jb) * jb * batch, st, &rec);
+  ck(qr_panel(R.mp, jb, W.at(j, j).p, W.ld, W.stride, tau + j, n, T + (j / PW) * PW * PW, strideT, Vp.p, Vp.ld,
+              Vp.stride, batch, st, R.split, R.gap, c.fault_word()));
+  if (c.prof.on) c.prof.end(rec, st);
+  c.stats.launches++;
+}
+
+// Householder QR panel by panel.  The chain (a panel, its reflector on the next panel's columns, the
+// next panel) runs on the high-priority side stream alone, so that no step of it waits for another
+// stream's event; the main stream updates the columns further right beside the next panel.
+static void geqrf_panelwise(Context& c, int mtot, int n, int m_top, Mat W, double* tau, double* T, int64_t strideT,
+                            int batch, bool top_tri) {
+  cudaStream_t ms = c.stream(), ss = c.side_stream();
+  const Mat none{nullptr, 0, 0};
+  if (n <= 2 * PW) ss = ms;  // nothing to update beside a panel
+  if (ss != ms) {
+    ck(cudaEventRecord(c.event(0), ms));
+    ck(cudaStreamWaitEvent(ss, c.event(0), 0));
+  }
+  bool rest = false;  // an update of the main stream that the next step on the side stream needs
+  for (int j = 0; j < n; j += PW) {
+    factor_panel(c, mtot, n, m_top, top_tri, j, W, tau, T, strideT, none, batch, ss);
+    const int nc = n - j - PW, jn = std::min(PW, nc);
+    if (nc <= 0) break;
+    const PanelRows R = panel_rows(mtot, m_top, top_tri, j, PW);
+    const double* Tj = T + (j / PW) * PW * PW;
+    if (nc > jn) ck(cudaEventRecord(c.event(0), ss));
+    if (rest) ck(cudaStreamWaitEvent(ss, c.event(1), 0));
+    apply_panel(c, R, PW, jn, W.at(j, j), Tj, strideT, 1, W.at(j, j + PW), batch, ss);
+    rest = nc > jn;
+    if (rest) {
+      ck(cudaStreamWaitEvent(ms, c.event(0), 0));
+      apply_panel(c, R, PW, nc - jn, W.at(j, j), Tj, strideT, 1, W.at(j, j + PW + jn), batch, ms);
+      ck(cudaEventRecord(c.event(1), ms));
+    }
+  }
+  if (ss != ms) {
+    ck(cudaEventRecord(c.event(0), ss));
+    ck(cudaStreamWaitEvent(ms, c.event(0), 0));
+  }
+}
+
 // Householder QR in 128-column blocks of four 32-column panels.  Inside a block each panel
 // updates only the block's remaining columns (rank-32); the trailing columns take one
 // rank-128 update per block, C -= V_B (T_B^T (V_B^T C)), whose GEMMs have K = rows and
@@ -368,6 +436,7 @@ void geqrf(Context& c, int mtot, int n, int m_top, Mat W, double* tau, double* T
   const int npan = (n + PW - 1) / PW;
   const int64_t ldv = (mtot + 1) / 2 * 2;
   const int64_t strideT = static_cast<int64_t>(npan) * PW * PW;
+  if (panelwise(mtot, n, batch, true)) return geqrf_panelwise(c, mtot, n, m_top, W, tau, T, strideT, batch, top_tri);
   Mat Vp{c.buf("qr_v2", static_cast<size_t>(ldv) * PW * batch), ldv, ldv * PW};
   Mat Pp{c.buf("qr_p", static_cast<size_t>(PW) * QB * batch), PW, static_cast<int64_t>(PW) * QB};
   Mat VB{c.buf("qr_vb", static_cast<size_t>(ldv) * QB * batch), ldv, ldv * QB};
@@ -381,14 +450,16 @@ void geqrf(Context& c, int mtot, int n, int m_top, Mat W, double* tau, double* T
       const int jb = std::min(PW, n - j);
       const int pj = j / PW;
       const PanelRows R = panel_rows(mtot, m_top, top_tri, j, jb);
-      Profiler::Rec rec;
-      if (c.prof.on) c.prof.begin(1, 2.0 * R.mp * static_cast<double>(jb) * jb * batch, st, &rec);
-      ck(qr_panel(R.mp, jb, W.at(j, j).p, W.ld, W.stride, tau + j, n, T + pj * PW * PW, strideT, Vp.p, Vp.ld,
-                  Vp.stride, batch, st, R.split, R.gap, c.fault_word()));
-      if (c.prof.on) c.prof.end(rec, st);
-      c.stats.launches++;
       const int nc = jend - j - jb;
+      // the panel on the block's other columns in one launch, 8 us where three products take 35 at
+      // least; a large batch is past latency, and the products' 10 TF/s beat its 4.6
+      const bool one = reflect_applies(R.mp) && static_cast<double>(R.mp) * nc * batch <= 1.2e6;
+      factor_panel(c, mtot, n, m_top, top_tri, j, W, tau, T, strideT, one ? Mat{nullptr, 0, 0} : Vp, batch, st);
       if (nc <= 0) continue;
+      if (one) {
+        apply_panel(c, R, jb, nc, W.at(j, j), T + pj * PW * PW, strideT, 1, W.at(j, j + jb), batch, st);
+        continue;
+      }
       panel_vt_b(c, R, jb, nc, Vp, W.at(j, j + jb), Pp, batch, st);
       ck(apply_t(jb, nc, T + pj * PW * PW, strideT, Pp.p, Pp.ld, Pp.stride, 1, batch, st));
       c.stats.launches++;
@@ -438,6 +509,14 @@ static void apply_q_blocks(Context& c, int mtot, int n, int m_top, Mat W, const 
   const int npan = (n + PW - 1) / PW;
   const int64_t ldv = (mtot + 1) / 2 * 2;
   const int64_t strideT = static_cast<int64_t>(npan) * PW * PW;
+  if (width == QB && panelwise(mtot, ncols, batch, false)) {
+    for (int j = (npan - 1) * PW; j >= 0; j -= PW) {
+      const int jb = std::min(PW, n - j), c0 = from_diag ? j : 0;
+      apply_panel(c, panel_rows(mtot, m_top, top_tri, j, jb), jb, ncols - c0, W.at(j, j), T + (j / PW) * PW * PW,
+                  strideT, 0, C.at(j, c0), batch, c.stream());
+    }
+    return;
+  }
   const int bw = std::min(width, (n + PW - 1) / PW * PW);
   Mat VB{c.buf("qr_vb", static_cast<size_t>(ldv) * bw * batch), ldv, ldv * bw};
   Mat TB{c.buf("qr_tb", static_cast<size_t>(bw) * bw * batch), bw, static_cast<int64_t>(bw) * bw};

@@ -672,7 +672,7 @@ __global__ void __launch_bounds__(NW * 32, 1) qr_panel_reg_kernel(PanelArgs p) {
       if (l0 + 8 * i >= nloc) continue;
       const int r = r0 + l0 + 8 * i;
       col[ro[i]] = a[i][j];
-      vcol[8 * i] = r > c ? a[i][j] : (r == c ? 1.0 : 0.0);
+      if (p.V) vcol[8 * i] = r > c ? a[i][j] : (r == c ? 1.0 : 0.0);
     }
   }
   if (rank == CL - 1 && warp == 1) {
@@ -848,6 +848,8 @@ bool reg_config(int m, int batch, int maxcl, int* cl, int* nw) {
 }
 
 }  // namespace
+
+int panel_cluster_max() { return max_cluster(); }
 
 int qr_panel_config(int m, int w) {
   const int maxcl = max_cluster();
