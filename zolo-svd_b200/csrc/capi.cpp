@@ -775,9 +775,7 @@ int zolo_dtrtri_dev(zolo_handle_t h, int n, const double* dL, int64_t ldl, doubl
   if (n == 0) return 0;
   return guarded(h, [&](Context& c) {
     zolo::Mat L{const_cast<double*>(dL), ldl, 0}, Y{dY, ldy, 0};
-    zolo::DiagInv D{c.buf("dinv", static_cast<size_t>(zolo::nblocks(n)) * 4096), 0};
-    zolo::diag_inverses(c, n, L, 1, D);
-    zolo::trtri_lower(c, n, L, Y, 1, D);
+    zolo::trtri_lower(c, n, L, Y, 1);
     zolo::ck(cudaStreamSynchronize(c.stream()));
     return 0;
   });

@@ -111,13 +111,13 @@ cudaError_t reduce_sum(const double* partial, int count, double* out, cudaStream
 // ---- Cholesky / triangular (potrf.cu) ----
 // In-place lower Cholesky of nb x nb blocks (nb <= 64), batched; LAPACK INFO (+info_offset)
 // recorded in info[b]; when Dinv != nullptr the inverse of the factor goes to
-// Dinv + b*strideD (64 x 64, ld 64, zeros above the diagonal).
+// Dinv + b*strideD (nb x nb, ld ldd, zeros above the diagonal).
 cudaError_t potrf_leaf(int nb, double* A, int64_t lda, int64_t strideA, int batch, int* info,
-                       int info_offset, double* Dinv, int64_t strideD, cudaStream_t st);
+                       int info_offset, double* Dinv, int64_t ldd, int64_t strideD, cudaStream_t st);
 // Inverses of all 64 x 64 diagonal blocks of lower-triangular n x n matrices:
-// block kb of batch entry b -> Dinv + (b*nblk + kb)*4096, nblk = ceil(n/64).
-cudaError_t trtri_blocks(int n, const double* L, int64_t ldl, int64_t strideL, double* Dinv, int batch,
-                         cudaStream_t st);
+// block kb of batch entry b -> Dinv + b*strideD + kb*blk, ld ldd.
+cudaError_t trtri_blocks(int n, const double* L, int64_t ldl, int64_t strideL, double* Dinv, int64_t ldd, int64_t blk,
+                         int64_t strideD, int batch, cudaStream_t st);
 
 // ---- Householder QR panel (qr.cu) ----
 // Factor the m x w panel of each batch entry (w <= 32) in place: V below the

@@ -193,7 +193,7 @@ static void potrf_rec(Context& c, int n, Mat A, int batch, int* dinfo, int off, 
   if (n <= NB) {
     Profiler::Rec rec;
     if (c.prof.on) c.prof.begin(2, static_cast<double>(n) * n * n / 3.0 * batch, c.stream(), &rec);
-    ck(potrf_leaf(n, A.p, A.ld, A.stride, batch, dinfo, off, D.block(off / NB), D.stride, c.stream()));
+    ck(potrf_leaf(n, A.p, A.ld, A.stride, batch, dinfo, off, D.block(off / NB), NB, D.stride, c.stream()));
     if (c.prof.on) c.prof.end(rec, c.stream());
     c.stats.launches++;
     return;
@@ -220,44 +220,48 @@ void potrf(Context& c, int n, Mat A, int batch, int* dinfo, DiagInv D) {
   potrf_rec(c, n, A, batch, dinfo, 0, D);
 }
 
-// Cholesky and the inverse of its factor together: with L11 and Y11 = L11^{-1} from the
-// first half, L21 = A21 Y11^T is one GEMM (no recursive triangular solve), then
-// A22 -= L21 L21^T, the second half, and Y21 = -Y22 (L21 Y11).  n^3/3 + n^3/3 flops, as
-// Cholesky plus triangular inverse, in about half the launches.
-static void potrf_inv_rec(Context& c, int n, Mat A, Mat Y, int batch, int* dinfo, int off, DiagInv D, Mat Tmp) {
+// Scratch of a node's n2 x n1 block (even leading dimension), and the most that any split of n rows
+// takes: even(n2) n1 <= (n2 + 1) n1 with n1 + n2 = n.
+static Mat block21(double* p, int n1, int n2) {
+  const int64_t ld = (n2 + 1) / 2 * 2;
+  return Mat{p, ld, ld * n1};
+}
+static size_t block21_elems(int n) { return static_cast<size_t>(n / 2 + 1) * (n / 2 + 1); }
+
+// Cholesky and the inverse of its factor together: with Y11 = L11^{-1} from the first half,
+// L21 = A21 Y11^T is one GEMM (no recursive triangular solve) into Tmp, A21 <- L21 Y11, then
+// A22 -= L21 L21^T, the second half, and Y21 = -Y22 A21.  n^3/3 + n^3/3 flops, as Cholesky plus
+// triangular inverse, in four launches a node; only Y is complete at the end.
+static void potrf_inv_rec(Context& c, int n, Mat A, Mat Y, int batch, int* dinfo, int off, double* tmp) {
   if (n <= NB) {
     Profiler::Rec rec;
     if (c.prof.on) c.prof.begin(2, static_cast<double>(n) * n * n / 3.0 * batch, c.stream(), &rec);
-    ck(potrf_leaf(n, A.p, A.ld, A.stride, batch, dinfo, off, D.block(off / NB), D.stride, c.stream()));
+    ck(potrf_leaf(n, A.p, A.ld, A.stride, batch, dinfo, off, Y.p, Y.ld, Y.stride, c.stream()));
     if (c.prof.on) c.prof.end(rec, c.stream());
-    ck(scale_copy(n, n, 1.0, D.block(off / NB), NB, D.stride, Y.p, Y.ld, Y.stride, batch, 0.0, c.stream()));
-    c.stats.launches += 2;
+    c.stats.launches++;
     return;
   }
   const int n1 = split_point(n), n2 = n - n1;
-  potrf_inv_rec(c, n1, A, Y, batch, dinfo, off, D, Tmp);
-  // L21 = A21 Y11^T: Y11^T is upper triangular (k up to the column)
-  ck(scale_copy(n2, n1, 1.0, A.at(n1, 0).p, A.ld, A.stride, Tmp.p, Tmp.ld, Tmp.stride, batch, 0.0, c.stream()));
-  c.stats.launches++;
-  gemm(c, 0, 1, n2, n1, n1, 1.0, Tmp, Y, 0.0, A.at(n1, 0), batch, nullptr, 0, 0, nullptr, 2);
-  // A22 -= L21 L21^T (lower)
-  gemm(c, 0, 1, n2, n2, n1, -1.0, A.at(n1, 0), A.at(n1, 0), 1.0, A.at(n1, n1), batch, nullptr, 1, 0);
-  potrf_inv_rec(c, n2, A.at(n1, n1), Y.at(n1, n1), batch, dinfo, off + n1, D, Tmp);
-  // Y21 = -Y22 (L21 Y11): Y11 lower (k from the column), Y22 lower (k up to the row)
-  gemm(c, 0, 0, n2, n1, n1, 1.0, A.at(n1, 0), Y, 0.0, Tmp, batch, nullptr, 0, 1);
-  gemm(c, 0, 0, n2, n1, n2, -1.0, Y.at(n1, n1), Tmp, 0.0, Y.at(n1, 0), batch, nullptr, 0, 0, nullptr, 1);
+  potrf_inv_rec(c, n1, A, Y, batch, dinfo, off, tmp);
+  const Mat Tmp = block21(tmp, n1, n2);
+  // Y11^T is upper triangular (k up to the column), Y11 lower (k from the column)
+  gemm(c, 0, 1, n2, n1, n1, 1.0, A.at(n1, 0), Y, 0.0, Tmp, batch, nullptr, 0, 0, nullptr, 2);
+  gemm(c, 0, 0, n2, n1, n1, 1.0, Tmp, Y, 0.0, A.at(n1, 0), batch, nullptr, 0, 1);
+  gemm(c, 0, 1, n2, n2, n1, -1.0, Tmp, Tmp, 1.0, A.at(n1, n1), batch, nullptr, 1, 0);
+  potrf_inv_rec(c, n2, A.at(n1, n1), Y.at(n1, n1), batch, dinfo, off + n1, tmp);
+  // Y22 lower: k up to the row
+  gemm(c, 0, 0, n2, n1, n2, -1.0, Y.at(n1, n1), A.at(n1, 0), 0.0, Y.at(n1, 0), batch, nullptr, 0, 0, nullptr, 1);
 }
 
-void potrf_inv(Context& c, int n, Mat A, Mat Y, int batch, int* dinfo, DiagInv D) {
+void potrf_inv(Context& c, int n, Mat A, Mat Y, int batch, int* dinfo) {
   ck(set_identity(n, n, Y.p, Y.ld, Y.stride, batch, 0.0, c.stream()));  // zero upper triangle
   c.stats.launches++;
-  const int64_t ldt = (n + 1) / 2 * 2;
-  Mat Tmp{c.buf("potrf_inv_tmp", static_cast<size_t>(ldt) * n * batch), ldt, ldt * n};
-  potrf_inv_rec(c, n, A, Y, batch, dinfo, 0, D, Tmp);
+  potrf_inv_rec(c, n, A, Y, batch, dinfo, 0, c.buf("potrf_inv_tmp", block21_elems(n) * batch));
 }
 
 void diag_inverses(Context& c, int n, Mat L, int batch, DiagInv D) {
-  ck(trtri_blocks(n, L.p, L.ld, L.stride, D.p, batch, c.stream()));
+  ck(trtri_blocks(n, L.p, L.ld, L.stride, D.p, NB, NB * NB, static_cast<int64_t>(nblocks(n)) * NB * NB, batch,
+                  c.stream()));
   c.stats.launches++;
 }
 
@@ -285,6 +289,37 @@ void trsm_rln(Context& c, int m, int n, Mat L, Mat X, Mat Y, int batch, DiagInv 
   trsm_rln(c, m, n1, L, X, Y, batch, D, k0);
 }
 
+// Level by level from the inverses of the 64 x 64 diagonal blocks: at block size s the blocks
+// below the diagonal of all pairs of one matrix are two launches (batched over the pairs; a
+// batch of matrices takes the pairs one after another), where the recursion by nodes took two a
+// pair: 8 products instead of 30 in the chain at n = 1024.
+void trtri_lower(Context& c, int n, Mat L, Mat Y, int batch) {
+  ck(set_identity(n, n, Y.p, Y.ld, Y.stride, batch, 0.0, c.stream()));  // zero upper triangle
+  ck(trtri_blocks(n, L.p, L.ld, L.stride, Y.p, Y.ld, NB * (Y.ld + 1), Y.stride, batch, c.stream()));
+  c.stats.launches += 2;
+  if (n <= NB) return;
+  double* tmp = c.buf("trtri_tmp", block21_elems(n) * batch);
+  // Y21 = -Y22 (L21 Y11) of `count` pairs from row o on, s + t rows each
+  auto pairs = [&](int o, int s, int t, int count) {
+    auto view = [&](Mat m, int i, int j) {
+      m = m.at(o + i, o + j);
+      if (count > 1) m.stride = 2 * s * (m.ld + 1);
+      return m;
+    };
+    const int nb = count > 1 ? count : batch;
+    const Mat P = block21(tmp, s, t);
+    gemm(c, 0, 0, t, s, s, 1.0, view(L, s, 0), view(Y, 0, 0), 0.0, P, nb, nullptr, 0, 1);
+    gemm(c, 0, 0, t, s, t, -1.0, view(Y, s, s), P, 0.0, view(Y, s, 0), nb, nullptr, 0, 0, nullptr, 1);
+  };
+  for (int s = NB; s < n; s *= 2) {
+    const int full = n / (2 * s), rest = n - full * 2 * s;
+    if (batch == 1 && full > 1) pairs(0, s, s, full);
+    else
+      for (int q = 0; q < full; ++q) pairs(q * 2 * s, s, s, 1);
+    if (rest > s) pairs(full * 2 * s, s, rest - s, 1);
+  }
+}
+
 // Rows of panel j (columns j .. j + jb - 1) in the mtot x n matrix: `mp`
 // logical rows, of which the first `split` start at row j and the rest follow
 // after `gap` skipped rows (gap = 0: one window).
@@ -292,28 +327,6 @@ struct PanelRows {
   int mp, split;
   int64_t gap;
 };
-
-static void trtri_rec(Context& c, int n, Mat L, Mat Y, int batch, DiagInv D, int k0, Mat Tmp) {
-  if (n <= NB) {
-    ck(scale_copy(n, n, 1.0, D.block(k0), NB, D.stride, Y.p, Y.ld, Y.stride, batch, 0.0, c.stream()));
-    c.stats.launches++;
-    return;
-  }
-  const int n1 = split_point(n), n2 = n - n1;
-  trtri_rec(c, n1, L, Y, batch, D, k0, Tmp);
-  trtri_rec(c, n2, L.at(n1, n1), Y.at(n1, n1), batch, D, k0 + n1 / NB, Tmp);
-  // Y21 = -Y22 (L21 Y11): Y11 lower (k from the output column), Y22 lower (k up to the row)
-  gemm(c, 0, 0, n2, n1, n1, 1.0, L.at(n1, 0), Y, 0.0, Tmp, batch, nullptr, 0, 1);
-  gemm(c, 0, 0, n2, n1, n2, -1.0, Y.at(n1, n1), Tmp, 0.0, Y.at(n1, 0), batch, nullptr, 0, 0, nullptr, 1);
-}
-
-void trtri_lower(Context& c, int n, Mat L, Mat Y, int batch, DiagInv D) {
-  ck(set_identity(n, n, Y.p, Y.ld, Y.stride, batch, 0.0, c.stream()));  // zero upper triangle
-  c.stats.launches++;
-  const int64_t ldt = (n + 1) / 2 * 2;
-  Mat Tmp{c.buf("trtri_tmp", static_cast<size_t>(ldt) * n * batch), ldt, ldt * n};
-  trtri_rec(c, n, L, Y, batch, D, 0, Tmp);
-}
 
 static inline PanelRows panel_rows(int mtot, int m_top, bool top_tri, int j, int jb) {
   const int hi = m_top >= 0 ? std::min(mtot, m_top + j + jb) : mtot;

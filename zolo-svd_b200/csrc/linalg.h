@@ -40,19 +40,19 @@ int oz_status(Context& c);
 // Lower Cholesky in place (n x n), recursive; info[b] > 0 on failure (LAPACK convention).
 // Dinv receives the inverses of the diagonal blocks of L (used by the solves below).
 void potrf(Context& c, int n, Mat A, int batch, int* dinfo, DiagInv Dinv);
-// Cholesky A = L L^T (lower, in place) and Y = L^{-1} (lower, upper triangle zero) together;
-// D receives the leaves' diagonal-block inverses, dinfo LAPACK INFO per batch entry.
-void potrf_inv(Context& c, int n, Mat A, Mat Y, int batch, int* dinfo, DiagInv D);
+// Y = L^{-1} (lower, upper triangle zero) of the Cholesky factor A = L L^T; A is destroyed, dinfo
+// receives LAPACK INFO per batch entry.
+void potrf_inv(Context& c, int n, Mat A, Mat Y, int batch, int* dinfo);
 // Dinv for a lower-triangular L that did not come from potrf.
 void diag_inverses(Context& c, int n, Mat L, int batch, DiagInv Dinv);
 // Y = X L^{-T}  (X m x n is destroyed; L's diagonal block k has inverse Dinv.block(k0 + k))
 void trsm_rlt(Context& c, int m, int n, Mat L, Mat X, Mat Y, int batch, DiagInv Dinv, int k0 = 0);
 // Y = X L^{-1}
 void trsm_rln(Context& c, int m, int n, Mat L, Mat X, Mat Y, int batch, DiagInv Dinv, int k0 = 0);
-// Y = L^{-1} (lower triangular; Y's strictly upper triangle is set to zero), recursively:
-// Y21 = -Y22 (L21 Y11), each product skipping the zero triangle of its triangular
-// operand (n^3/3 flops); the 64 x 64 diagonal blocks are Dinv's.
-void trtri_lower(Context& c, int n, Mat L, Mat Y, int batch, DiagInv Dinv);
+// Y = L^{-1} (lower triangular; Y's strictly upper triangle is set to zero), blocks merged pair by
+// pair: Y21 = -Y22 (L21 Y11), each product skipping the zero triangle of its triangular operand
+// (n^3/3 flops).
+void trtri_lower(Context& c, int n, Mat L, Mat Y, int batch);
 
 // Householder QR (in place, panels of 32) of the mtot x n matrices W.  With
 // `m_top` >= 0 the matrix is the stack [X (m_top rows); D] where D is upper

@@ -112,7 +112,8 @@ cudaError_t trsm_rlt_static(int m, int n, const double* L, int64_t ldl, double* 
 cudaError_t potrf_static(int n, double* A, int64_t lda, int off, double* tmp, double* dinv, int* info,
                          cudaStream_t st) {
   if (n <= kLeafN)
-    return potrf_leaf(n, A, lda, 0, 1, info, off, dinv + static_cast<int64_t>(off / kLeafN) * 4096, 0, st);
+    return potrf_leaf(n, A, lda, 0, 1, info, off, dinv + static_cast<int64_t>(off / kLeafN) * 4096, kLeafN, 0,
+                      st);
   const int n1 = split_at(n), n2 = n - n1;
   cudaError_t e = potrf_static(n1, A, lda, off, tmp, dinv, info, st);
   if (e != cudaSuccess) return e;

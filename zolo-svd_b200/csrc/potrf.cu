@@ -180,7 +180,7 @@ ZDEV void load_leaf(int nb, const double* A, int64_t lda, double* a, double* x) 
 }
 
 __global__ void __launch_bounds__(PT) potrf_leaf_kernel(int nb, double* A, int64_t lda, int64_t strideA, int* info,
-                                                        int info_offset, double* Dinv, int64_t strideD) {
+                                                        int info_offset, double* Dinv, int64_t ldd, int64_t strideD) {
   extern __shared__ double sm[];
   double* a = sm;
   double* x = sm + LEAF * LDS;
@@ -234,14 +234,15 @@ __global__ void __launch_bounds__(PT) potrf_leaf_kernel(int nb, double* A, int64
   double* Db = Dinv + blockIdx.x * strideD;
   for (int e = threadIdx.x; e < LEAF * LEAF; e += PT) {
     const int i = e & (LEAF - 1), j = e >> 6;
-    if (i < nb && j < nb) Db[i + j * LEAF] = x[i + j * LDS];
+    if (i < nb && j < nb) Db[i + j * ldd] = x[i + j * LDS];
   }
 }
 
 // Inverses of the diagonal blocks of a lower-triangular n x n matrix:
-// block kb (rows/cols kb*64 ..) of batch entry b goes to Dinv + (b*nblk + kb)*64*64.
+// block kb (rows/cols kb*64 ..) of batch entry b goes to Dinv + b*strideD + kb*blk (ld ldd).
 __global__ void __launch_bounds__(PT) trtri_blocks_kernel(int n, const double* L, int64_t ldl, int64_t strideL,
-                                                          double* Dinv, int nblk) {
+                                                          double* Dinv, int64_t ldd, int64_t blk,
+                                                          int64_t strideD) {
   extern __shared__ double sm[];
   double* l = sm;
   double* x = sm + LEAF * LDS;
@@ -253,10 +254,10 @@ __global__ void __launch_bounds__(PT) trtri_blocks_kernel(int n, const double* L
   if (warp < LEAF / LB) invert_block(l, x, warp * LB);
   __syncthreads();
   merge_inverse(l, x);
-  double* Db = Dinv + (static_cast<int64_t>(b) * nblk + kb) * LEAF * LEAF;
+  double* Db = Dinv + b * strideD + kb * blk;
   for (int e = threadIdx.x; e < LEAF * LEAF; e += PT) {
     const int i = e & (LEAF - 1), j = e >> 6;
-    if (i < nb && j < nb) Db[i + j * LEAF] = x[i + j * LDS];
+    if (i < nb && j < nb) Db[i + j * ldd] = x[i + j * LDS];
   }
 }
 
@@ -265,7 +266,7 @@ constexpr int SMEM_BYTES = 2 * LEAF * LDS * 8;
 }  // namespace
 
 cudaError_t potrf_leaf(int nb, double* A, int64_t lda, int64_t strideA, int batch, int* info, int info_offset,
-                       double* Dinv, int64_t strideD, cudaStream_t st) {
+                       double* Dinv, int64_t ldd, int64_t strideD, cudaStream_t st) {
   if (nb <= 0 || batch <= 0) return cudaSuccess;
   if (nb > LEAF) return cudaErrorInvalidValue;
   static std::atomic<int> attr_set[kMaxDevices];
@@ -273,12 +274,12 @@ cudaError_t potrf_leaf(int nb, double* A, int64_t lda, int64_t strideA, int batc
     return cudaFuncSetAttribute(potrf_leaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   });
   if (attr != cudaSuccess) return attr;
-  potrf_leaf_kernel<<<batch, PT, SMEM_BYTES, st>>>(nb, A, lda, strideA, info, info_offset, Dinv, strideD);
+  potrf_leaf_kernel<<<batch, PT, SMEM_BYTES, st>>>(nb, A, lda, strideA, info, info_offset, Dinv, ldd, strideD);
   return cudaGetLastError();
 }
 
-cudaError_t trtri_blocks(int n, const double* L, int64_t ldl, int64_t strideL, double* Dinv, int batch,
-                         cudaStream_t st) {
+cudaError_t trtri_blocks(int n, const double* L, int64_t ldl, int64_t strideL, double* Dinv, int64_t ldd, int64_t blk,
+                         int64_t strideD, int batch, cudaStream_t st) {
   if (n <= 0 || batch <= 0) return cudaSuccess;
   static std::atomic<int> attr_set[kMaxDevices];
   const cudaError_t attr = once_per_device(attr_set, [] {
@@ -286,7 +287,7 @@ cudaError_t trtri_blocks(int n, const double* L, int64_t ldl, int64_t strideL, d
   });
   if (attr != cudaSuccess) return attr;
   const int nblk = (n + LEAF - 1) / LEAF;
-  trtri_blocks_kernel<<<dim3(nblk, batch), PT, SMEM_BYTES, st>>>(n, L, ldl, strideL, Dinv, nblk);
+  trtri_blocks_kernel<<<dim3(nblk, batch), PT, SMEM_BYTES, st>>>(n, L, ldl, strideL, Dinv, ldd, blk, strideD);
   return cudaGetLastError();
 }
 
