@@ -172,6 +172,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) dgemm_kernel(KParams kp) {
   // C reads overlap the A/B copies instead of following them.  C is pre-scaled by
   // beta/alpha (exact for alpha = +-1) and the epilogue then writes alpha * acc.
   const bool preload = kp.preload;
+  dependency_wait();
   if (preload) {
     const double* Cb = p.C + static_cast<int64_t>(bz) * p.strideC;
     const double sc = p.beta / p.alpha;
@@ -255,6 +256,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) dgemm_kernel(KParams kp) {
     }
   }
   cp_async_wait<0>();
+  release_dependents();
 
   // ---- epilogue ----
   if (kp.splitk > 1) {
@@ -340,23 +342,8 @@ cudaError_t launch_t(const KParams& kp, dim3 grid, cudaStream_t st) {
                                 C::smem(TA, TB));
   });
   if (attr != cudaSuccess) return attr;
-  if (kp.splitk <= 1) {
-    dgemm_kernel<C, TA, TB, V16><<<grid, C::NT, C::smem(TA, TB), st>>>(kp);
-    return cudaGetLastError();
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(C::NT, 1, 1);
-  cfg.dynamicSmemBytes = C::smem(TA, TB);
-  cfg.stream = st;
-  cudaLaunchAttribute la[1];
-  la[0].id = cudaLaunchAttributeClusterDimension;
-  la[0].val.clusterDim.x = 1;
-  la[0].val.clusterDim.y = kp.splitk;
-  la[0].val.clusterDim.z = 1;
-  cfg.attrs = la;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, dgemm_kernel<C, TA, TB, V16>, kp);
+  return launch_dependent(dgemm_kernel<C, TA, TB, V16>, grid, dim3(C::NT), C::smem(TA, TB), st, dim3(1, kp.splitk, 1),
+                          kp);
 }
 
 template <class C, bool V16>

@@ -187,6 +187,7 @@ __global__ void __launch_bounds__(PT) potrf_leaf_kernel(int nb, double* A, int64
   double* Ab = A + blockIdx.x * strideA;
   const int warp = threadIdx.x >> 5;
   __shared__ __align__(16) double piv[4 * LB];
+  dependency_wait();
   load_leaf(nb, Ab, lda, a, x);
   const int n16 = (nb + LB - 1) / LB * LB;  // identity blocks past nb need no elimination
   for (int k0 = 0; k0 < n16; k0 += LB) {
@@ -228,6 +229,7 @@ __global__ void __launch_bounds__(PT) potrf_leaf_kernel(int nb, double* A, int64
     if (i < nb && j <= i) Ab[i + j * lda] = a[i + j * LDS];
     if (i >= n16 && i == j) x[i + j * LDS] = 1.0;
   }
+  release_dependents();
   if (!Dinv) return;
   __syncthreads();
   merge_inverse(a, x);
@@ -249,6 +251,7 @@ __global__ void __launch_bounds__(PT) trtri_blocks_kernel(int n, const double* L
   const int kb = blockIdx.x, b = blockIdx.y;
   const int o = kb * LEAF;
   const int nb = min(LEAF, n - o);
+  dependency_wait();
   load_leaf(nb, L + b * strideL + o + static_cast<int64_t>(o) * ldl, ldl, l, x);
   const int warp = threadIdx.x >> 5;
   if (warp < LEAF / LB) invert_block(l, x, warp * LB);
@@ -274,8 +277,8 @@ cudaError_t potrf_leaf(int nb, double* A, int64_t lda, int64_t strideA, int batc
     return cudaFuncSetAttribute(potrf_leaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   });
   if (attr != cudaSuccess) return attr;
-  potrf_leaf_kernel<<<batch, PT, SMEM_BYTES, st>>>(nb, A, lda, strideA, info, info_offset, Dinv, ldd, strideD);
-  return cudaGetLastError();
+  return launch_dependent(potrf_leaf_kernel, dim3(batch), dim3(PT), SMEM_BYTES, st, dim3(1), nb, A, lda, strideA, info,
+                          info_offset, Dinv, ldd, strideD);
 }
 
 cudaError_t trtri_blocks(int n, const double* L, int64_t ldl, int64_t strideL, double* Dinv, int64_t ldd, int64_t blk,
@@ -287,8 +290,8 @@ cudaError_t trtri_blocks(int n, const double* L, int64_t ldl, int64_t strideL, d
   });
   if (attr != cudaSuccess) return attr;
   const int nblk = (n + LEAF - 1) / LEAF;
-  trtri_blocks_kernel<<<dim3(nblk, batch), PT, SMEM_BYTES, st>>>(n, L, ldl, strideL, Dinv, ldd, blk, strideD);
-  return cudaGetLastError();
+  return launch_dependent(trtri_blocks_kernel, dim3(nblk, batch), dim3(PT), SMEM_BYTES, st, dim3(1), n, L, ldl, strideL,
+                          Dinv, ldd, blk, strideD);
 }
 
 }  // namespace zolo

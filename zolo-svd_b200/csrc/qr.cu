@@ -631,14 +631,6 @@ __global__ void __launch_bounds__(NW * 32, 1) qr_panel_reg_kernel(PanelArgs p) {
   int64_t ro[RN];
 #pragma unroll
   for (int i = 0; i < RN; ++i) ro[i] = 8 * i + (r0 + l0 + 8 * i >= p.split ? p.gap : 0);
-  double a[RN][8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const bool in = 2 * t + (j & 1) + 8 * (j >> 1) < w;
-    const double* col = A + ((j & 1) + 8 * (j >> 1)) * lda;
-#pragma unroll
-    for (int i = 0; i < RN; ++i) a[i][j] = (in && l0 + 8 * i < nloc) ? col[ro[i]] : 0.0;
-  }
   if (CL > 1) {
     if (threadIdx.x == 0) {
       S.abort = 0;
@@ -652,6 +644,15 @@ __global__ void __launch_bounds__(NW * 32, 1) qr_panel_reg_kernel(PanelArgs p) {
     // every CTA of the cluster runs, its barriers ready, before the first send to it
     cluster_sync_all();
   }
+  dependency_wait();
+  double a[RN][8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const bool in = 2 * t + (j & 1) + 8 * (j >> 1) < w;
+    const double* col = A + ((j & 1) + 8 * (j >> 1)) * lda;
+#pragma unroll
+    for (int i = 0; i < RN; ++i) a[i][j] = (in && l0 + 8 * i < nloc) ? col[ro[i]] : 0.0;
+  }
   if (!panel_factor<NW, RN>(a, S, w, r0, nloc, rank, CL)) {
     if (threadIdx.x == 0 && p.status) {
       *static_cast<volatile int*>(p.status) = 911;
@@ -660,6 +661,7 @@ __global__ void __launch_bounds__(NW * 32, 1) qr_panel_reg_kernel(PanelArgs p) {
     cluster_sync_all();  // no CTA leaves while others may still send to it
     return;
   }
+  release_dependents();
   double* V = p.V + b * p.strideV + r0 + l0 + 2 * t * p.ldv;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
@@ -781,18 +783,7 @@ cudaError_t launch_reg(const PanelArgs& pa, int cl, int batch, cudaStream_t st) 
     return cudaFuncSetAttribute(qr_panel_reg_kernel<NW, RN>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   });
   if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cl, batch, 1);
-  cfg.blockDim = dim3(NW * 32, 1, 1);
-  cfg.stream = st;
-  cudaLaunchAttribute attr_l[1];
-  attr_l[0].id = cudaLaunchAttributeClusterDimension;
-  attr_l[0].val.clusterDim.x = cl;
-  attr_l[0].val.clusterDim.y = 1;
-  attr_l[0].val.clusterDim.z = 1;
-  cfg.attrs = attr_l;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, qr_panel_reg_kernel<NW, RN>, pa);
+  return launch_dependent(qr_panel_reg_kernel<NW, RN>, dim3(cl, batch, 1), dim3(NW * 32), 0, st, dim3(cl), pa);
 }
 
 // 16-CTA clusters are non-portable: use them only if the device can place one

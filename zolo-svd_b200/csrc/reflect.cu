@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(RT) reflect_kernel(ReflArgs p) {
       }
     }
   };
+  dependency_wait();
   fetch(Vs, V, p.ldv, RW, p.w);
   fetch(Cs, C + n0 * p.ldc, p.ldc, RN, min(RN, p.nc - n0));
   cp_async_commit();
@@ -179,6 +180,7 @@ __global__ void __launch_bounds__(RT) reflect_kernel(ReflArgs p) {
   }
   if (CL > 1) cluster.sync();
   else __syncthreads();
+  release_dependents();
   // ---- C - V P, 16 rows x 16 columns at a time ----
   for (int l0 = warp * 16; l0 < nloc; l0 += RT / 32 * 16) {
     double acc[2][4];
@@ -263,19 +265,8 @@ cudaError_t reflect(int m, int nc, int w, const double* V, int64_t ldv, int64_t 
     return cudaSuccess;
   });
   if (attr != cudaSuccess) return attr;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(cl * ((nc + RN - 1) / RN)), batch, 1);
-  cfg.blockDim = dim3(RT, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute la[1];
-  la[0].id = cudaLaunchAttributeClusterDimension;
-  la[0].val.clusterDim.x = cl;
-  la[0].val.clusterDim.y = 1;
-  la[0].val.clusterDim.z = 1;
-  cfg.attrs = la;
-  cfg.numAttrs = 1;
-  return a16 ? cudaLaunchKernelEx(&cfg, reflect_kernel<true>, p) : cudaLaunchKernelEx(&cfg, reflect_kernel<false>, p);
+  const dim3 grid(static_cast<unsigned>(cl * ((nc + RN - 1) / RN)), batch, 1);
+  return launch_dependent(a16 ? reflect_kernel<true> : reflect_kernel<false>, grid, dim3(RT), smem, st, dim3(cl), p);
 }
 
 }  // namespace zolo
