@@ -155,6 +155,8 @@ __global__ void combine_batch_kernel(int m, int n, double* X, int64_t ldx, int64
 // which leaves X_b unchanged and its error 0).
 __global__ void gate_batch_kernel(int batch, const double* err2_prev, const double* cond, double* row, int qr,
                                   double tol) {
+  dependency_wait();
+  release_dependents();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= batch) return;
   if (cond[b] != 0.0 && !(sqrt(err2_prev[b]) > tol)) {
@@ -166,6 +168,8 @@ __global__ void gate_batch_kernel(int batch, const double* err2_prev, const doub
 
 // G_b += d I
 __global__ void add_diag_batch_kernel(int n, double* G, int64_t ldg, int64_t sg, double d) {
+  dependency_wait();
+  release_dependents();
   double* Gb = G + blockIdx.y * sg;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     Gb[i + static_cast<int64_t>(i) * ldg] += d;
@@ -189,6 +193,8 @@ __global__ void symmetrize_batch_kernel(int n, double* B, int64_t ldb, int64_t s
 // B_b = A_b^T  (A m x n)
 __global__ void transpose_batch_kernel(int m, int n, const double* A, int64_t lda, int64_t sa, double* B,
                                        int64_t ldb, int64_t sb) {
+  dependency_wait();
+  release_dependents();
   __shared__ double tile[32][33];
   const double* Ab = A + blockIdx.z * sa;
   double* Bb = B + blockIdx.z * sb;
@@ -260,14 +266,12 @@ cudaError_t batch_combine(int m, int n, double* X, int64_t ldx, int64_t sx, cons
 cudaError_t batch_gate(int batch, const double* err2_prev, const double* cond, double* row, int qr, double tol,
                        cudaStream_t st) {
   if (batch <= 0) return cudaSuccess;
-  gate_batch_kernel<<<(batch + TPB - 1) / TPB, TPB, 0, st>>>(batch, err2_prev, cond, row, qr, tol);
-  return cudaGetLastError();
+  return launch_dependent(gate_batch_kernel, dim3((batch + TPB - 1) / TPB), dim3(TPB), 0, st, dim3(1), batch, err2_prev, cond, row, qr, tol);
 }
 
 cudaError_t batch_add_diag(int n, double* G, int64_t ldg, int64_t sg, int batch, double d, cudaStream_t st) {
   if (batch <= 0) return cudaSuccess;
-  add_diag_batch_kernel<<<dim3(blocks_for(n, 8), batch), TPB, 0, st>>>(n, G, ldg, sg, d);
-  return cudaGetLastError();
+  return launch_dependent(add_diag_batch_kernel, dim3(blocks_for(n, 8), batch), dim3(TPB), 0, st, dim3(1), n, G, ldg, sg, d);
 }
 
 cudaError_t batch_symmetrize(int n, double* B, int64_t ldb, int64_t sb, int batch, cudaStream_t st) {
@@ -281,8 +285,7 @@ cudaError_t batch_transpose(int m, int n, const double* A, int64_t lda, int64_t 
   if (batch <= 0 || m <= 0 || n <= 0) return cudaSuccess;
   if (batch > 65535) return cudaErrorInvalidValue;
   dim3 grid((m + 31) / 32, (n + 31) / 32, batch);
-  transpose_batch_kernel<<<grid, dim3(32, 8), 0, st>>>(m, n, A, lda, sa, B, ldb, sb);
-  return cudaGetLastError();
+  return launch_dependent(transpose_batch_kernel, grid, dim3(32, 8), 0, st, dim3(1), m, n, A, lda, sa, B, ldb, sb);
 }
 
 }  // namespace zolo

@@ -22,6 +22,8 @@ inline int grid_for(int64_t work, int per_block = TPB) {
 __global__ void scale_copy_kernel(int m, int n, double s, const double* __restrict__ src, int64_t lds,
                                   int64_t strideS, double* dst, int64_t ldd, int64_t strideD,
                                   double diag_add) {
+  dependency_wait();
+  release_dependents();
   const int b = blockIdx.y;
   const double* S = src + b * strideS;
   double* D = dst + b * strideD;
@@ -38,6 +40,8 @@ __global__ void scale_copy_kernel(int m, int n, double s, const double* __restri
 __global__ void form_stack_kernel(int m, int mpad, int n, const double* __restrict__ X, int64_t ldx, double* W,
                                   int64_t ldw, int64_t strideW, const double* s_vec, double s_scalar,
                                   int x_upper, int64_t strideX) {
+  dependency_wait();
+  release_dependents();
   const int b = blockIdx.y;
   X += b * strideX;
   double* Wb = W + b * strideW;
@@ -56,6 +60,8 @@ __global__ void form_stack_kernel(int m, int mpad, int n, const double* __restri
 
 __global__ void shift_lower_kernel(int n, const double* __restrict__ G, int64_t ldg, double* W,
                                    int64_t ldw, int64_t strideW, const double* c_vec) {
+  dependency_wait();
+  release_dependents();
   const int b = blockIdx.y;
   double* Wb = W + b * strideW;
   const double c = c_vec[b];
@@ -85,6 +91,8 @@ __device__ double block_sum(double v, double* sh) {
 }
 
 __global__ void frob2_kernel(int m, int n, const double* __restrict__ X, int64_t ldx, double* partial) {
+  dependency_wait();
+  release_dependents();
   __shared__ double sh[TPB / 32];
   const int64_t total = static_cast<int64_t>(m) * n;
   double s = 0.0;
@@ -99,6 +107,8 @@ __global__ void frob2_kernel(int m, int n, const double* __restrict__ X, int64_t
 }
 
 __global__ void reduce_sum_kernel(const double* partial, int count, double* out) {
+  dependency_wait();
+  release_dependents();
   __shared__ double sh[TPB / 32];
   double s = 0.0;
   for (int i = threadIdx.x; i < count; i += blockDim.x) s += partial[i];
@@ -107,6 +117,8 @@ __global__ void reduce_sum_kernel(const double* partial, int count, double* out)
 }
 
 __global__ void colsum_abs_kernel(int m, int n, const double* __restrict__ X, int64_t ldx, double* colsum) {
+  dependency_wait();
+  release_dependents();
   __shared__ double sh[TPB / 32];
   for (int j = blockIdx.x; j < n; j += gridDim.x) {
     double s = 0.0;
@@ -117,6 +129,8 @@ __global__ void colsum_abs_kernel(int m, int n, const double* __restrict__ X, in
 }
 
 __global__ void max_kernel(const double* v, int count, double* out) {
+  dependency_wait();
+  release_dependents();
   __shared__ double sh[TPB];
   double s = 0.0;
   for (int i = threadIdx.x; i < count; i += blockDim.x) s = fmax(s, v[i]);
@@ -133,6 +147,8 @@ __global__ void max_kernel(const double* v, int count, double* out) {
 __global__ void combine_kernel(int m, int n, double* X, int64_t ldx, const double* __restrict__ Z,
                                int64_t ldz, int64_t strideZ, int nz, double cx, double cz,
                                const double* __restrict__ cz_vec, double* partial) {
+  dependency_wait();
+  release_dependents();
   __shared__ double sh[TPB / 32];
   const int64_t total = static_cast<int64_t>(m) * n;
   double s = 0.0;
@@ -157,6 +173,8 @@ __global__ void combine_kernel(int m, int n, double* X, int64_t ldx, const doubl
 }
 
 __global__ void symmetrize_kernel(int n, double* B, int64_t ldb) {
+  dependency_wait();
+  release_dependents();
   const int64_t total = static_cast<int64_t>(n) * n;
   for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
        e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -171,6 +189,8 @@ __global__ void symmetrize_kernel(int n, double* B, int64_t ldb) {
 
 __global__ void transpose_kernel(int m, int n, const double* __restrict__ A, int64_t lda, double* B,
                                  int64_t ldb) {
+  dependency_wait();
+  release_dependents();
   __shared__ double tile[32][33];
   const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
   for (int jj = threadIdx.y; jj < 32; jj += blockDim.y) {
@@ -188,6 +208,8 @@ __global__ void transpose_kernel(int m, int n, const double* __restrict__ A, int
 // (both triangles written; only when `write`) and partial[block] = sum of (G - I)^2
 // over all entries.
 __global__ void ns_prepare_kernel(int n, double* G, int64_t ldg, int write, double* partial) {
+  dependency_wait();
+  release_dependents();
   __shared__ double sh[TPB / 32];
   const int64_t total = static_cast<int64_t>(n) * n;
   double s = 0.0;
@@ -209,6 +231,8 @@ __global__ void ns_prepare_kernel(int n, double* G, int64_t ldg, int write, doub
 
 // B(j, i) = B(i, j) for i > j: the lower triangle copied to the upper one
 __global__ void mirror_lower_kernel(int n, double* B, int64_t ldb) {
+  dependency_wait();
+  release_dependents();
   const int64_t total = static_cast<int64_t>(n) * n;
   for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
        e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -219,6 +243,8 @@ __global__ void mirror_lower_kernel(int n, double* B, int64_t ldb) {
 
 __global__ void copy_upper_kernel(int n, const double* __restrict__ A, int64_t lda, double scale, double* B,
                                   int64_t ldb) {
+  dependency_wait();
+  release_dependents();
   const int64_t total = static_cast<int64_t>(n) * n;
   for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
        e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -228,6 +254,8 @@ __global__ void copy_upper_kernel(int n, const double* __restrict__ A, int64_t l
 }
 
 __global__ void set_identity_kernel(int m, int n, double* Q, int64_t ldq, int64_t strideQ, double diag) {
+  dependency_wait();
+  release_dependents();
   double* Qb = Q + blockIdx.y * strideQ;
   const int64_t total = static_cast<int64_t>(m) * n;
   for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
@@ -238,6 +266,8 @@ __global__ void set_identity_kernel(int m, int n, double* Q, int64_t ldq, int64_
 }
 
 __global__ void add_diag_kernel(int n, double* A, int64_t lda, double d) {
+  dependency_wait();
+  release_dependents();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     A[i + i * lda] += d;
 }
@@ -311,9 +341,7 @@ cudaError_t get_diag(int n, const double* A, int64_t lda, double* d, cudaStream_
 cudaError_t scale_copy(int m, int n, double s, const double* src, int64_t lds, int64_t strideS, double* dst,
                        int64_t ldd, int64_t strideD, int batch, double diag_add, cudaStream_t st) {
   if (m <= 0 || n <= 0 || batch <= 0) return cudaSuccess;
-  scale_copy_kernel<<<dim3(grid_for(static_cast<int64_t>(m) * n), batch), TPB, 0, st>>>(
-      m, n, s, src, lds, strideS, dst, ldd, strideD, diag_add);
-  return cudaGetLastError();
+  return launch_dependent(scale_copy_kernel, dim3(grid_for(static_cast<int64_t>(m) * n), batch), dim3(TPB), 0, st, dim3(1), m, n, s, src, lds, strideS, dst, ldd, strideD, diag_add);
 }
 
 cudaError_t form_stack(int m, int mpad, int n, const double* X, int64_t ldx, double* W, int64_t ldw,
@@ -321,93 +349,76 @@ cudaError_t form_stack(int m, int mpad, int n, const double* X, int64_t ldx, dou
                        int x_upper, int64_t strideX) {
   if (n <= 0 || batch <= 0) return cudaSuccess;
   if (mpad < m) return cudaErrorInvalidValue;
-  form_stack_kernel<<<dim3(grid_for(static_cast<int64_t>(mpad + n) * n), batch), TPB, 0, st>>>(
-      m, mpad, n, X, ldx, W, ldw, strideW, s_vec, s_scalar, x_upper, strideX);
-  return cudaGetLastError();
+  return launch_dependent(form_stack_kernel, dim3(grid_for(static_cast<int64_t>(mpad + n) * n), batch), dim3(TPB), 0, st, dim3(1), m, mpad, n, X, ldx, W, ldw, strideW, s_vec, s_scalar, x_upper, strideX);
 }
 
 cudaError_t shift_lower(int n, const double* G, int64_t ldg, double* W, int64_t ldw, int64_t strideW,
                         const double* c_vec, int batch, cudaStream_t st) {
   if (n <= 0 || batch <= 0) return cudaSuccess;
-  shift_lower_kernel<<<dim3(grid_for(static_cast<int64_t>(n) * n), batch), TPB, 0, st>>>(n, G, ldg, W, ldw,
-                                                                                         strideW, c_vec);
-  return cudaGetLastError();
+  return launch_dependent(shift_lower_kernel, dim3(grid_for(static_cast<int64_t>(n) * n), batch), dim3(TPB), 0, st, dim3(1), n, G, ldg, W, ldw, strideW, c_vec);
 }
 
 cudaError_t reduce_sum(const double* partial, int count, double* out, cudaStream_t st) {
-  reduce_sum_kernel<<<1, TPB, 0, st>>>(partial, count, out);
-  return cudaGetLastError();
+  return launch_dependent(reduce_sum_kernel, dim3(1), dim3(TPB), 0, st, dim3(1), partial, count, out);
 }
 
 cudaError_t frob2(int m, int n, const double* X, int64_t ldx, double* partial, double* out, cudaStream_t st) {
   const int blocks = std::min(grid_for(static_cast<int64_t>(m) * n), 1024);
-  frob2_kernel<<<blocks, TPB, 0, st>>>(m, n, X, ldx, partial);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_dependent(frob2_kernel, dim3(blocks), dim3(TPB), 0, st, dim3(1), m, n, X, ldx, partial);
   if (e != cudaSuccess) return e;
   return reduce_sum(partial, blocks, out, st);
 }
 
 cudaError_t norm1(int m, int n, const double* X, int64_t ldx, double* colsum, double* out, cudaStream_t st) {
-  colsum_abs_kernel<<<std::min(n, 4096), TPB, 0, st>>>(m, n, X, ldx, colsum);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_dependent(colsum_abs_kernel, dim3(std::min(n, 4096)), dim3(TPB), 0, st, dim3(1), m, n, X, ldx, colsum);
   if (e != cudaSuccess) return e;
-  max_kernel<<<1, TPB, 0, st>>>(colsum, n, out);
-  return cudaGetLastError();
+  return launch_dependent(max_kernel, dim3(1), dim3(TPB), 0, st, dim3(1), colsum, n, out);
 }
 
 cudaError_t combine_update(int m, int n, double* X, int64_t ldx, const double* Z, int64_t ldz, int64_t strideZ,
                            int nz, double cx, double cz, const double* cz_vec, double* partial, double* err2,
                            cudaStream_t st) {
   const int blocks = std::min(grid_for(static_cast<int64_t>(m) * n), 1024);
-  combine_kernel<<<blocks, TPB, 0, st>>>(m, n, X, ldx, Z, ldz, strideZ, nz, cx, cz, cz_vec, partial);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_dependent(combine_kernel, dim3(blocks), dim3(TPB), 0, st, dim3(1), m, n, X, ldx, Z, ldz, strideZ, nz, cx, cz, cz_vec, partial);
   if (e != cudaSuccess) return e;
   return reduce_sum(partial, blocks, err2, st);
 }
 
 cudaError_t symmetrize(int n, double* B, int64_t ldb, cudaStream_t st) {
-  symmetrize_kernel<<<grid_for(static_cast<int64_t>(n) * n), TPB, 0, st>>>(n, B, ldb);
-  return cudaGetLastError();
+  return launch_dependent(symmetrize_kernel, dim3(grid_for(static_cast<int64_t>(n) * n)), dim3(TPB), 0, st, dim3(1), n, B, ldb);
 }
 
 cudaError_t transpose(int m, int n, const double* A, int64_t lda, double* B, int64_t ldb, cudaStream_t st) {
   dim3 grid((m + 31) / 32, (n + 31) / 32);
-  transpose_kernel<<<grid, dim3(32, 8), 0, st>>>(m, n, A, lda, B, ldb);
-  return cudaGetLastError();
+  return launch_dependent(transpose_kernel, grid, dim3(32, 8), 0, st, dim3(1), m, n, A, lda, B, ldb);
 }
 
 cudaError_t ns_prepare(int n, double* G, int64_t ldg, double* partial, double* err2, int write, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   const int blocks = static_cast<int>(std::min<int64_t>(grid_for(static_cast<int64_t>(n) * n), 1024));
-  ns_prepare_kernel<<<blocks, TPB, 0, st>>>(n, G, ldg, write, partial);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_dependent(ns_prepare_kernel, dim3(blocks), dim3(TPB), 0, st, dim3(1), n, G, ldg, write, partial);
   if (e != cudaSuccess) return e;
   return reduce_sum(partial, blocks, err2, st);
 }
 
 cudaError_t copy_upper(int n, const double* A, int64_t lda, double scale, double* B, int64_t ldb, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  copy_upper_kernel<<<grid_for(static_cast<int64_t>(n) * n), TPB, 0, st>>>(n, A, lda, scale, B, ldb);
-  return cudaGetLastError();
+  return launch_dependent(copy_upper_kernel, dim3(grid_for(static_cast<int64_t>(n) * n)), dim3(TPB), 0, st, dim3(1), n, A, lda, scale, B, ldb);
 }
 
 cudaError_t mirror_lower(int n, double* B, int64_t ldb, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  mirror_lower_kernel<<<grid_for(static_cast<int64_t>(n) * n), TPB, 0, st>>>(n, B, ldb);
-  return cudaGetLastError();
+  return launch_dependent(mirror_lower_kernel, dim3(grid_for(static_cast<int64_t>(n) * n)), dim3(TPB), 0, st, dim3(1), n, B, ldb);
 }
 
 cudaError_t set_identity(int m, int n, double* Q, int64_t ldq, int64_t strideQ, int batch, double diag,
                          cudaStream_t st) {
   if (m <= 0 || n <= 0 || batch <= 0) return cudaSuccess;
-  set_identity_kernel<<<dim3(grid_for(static_cast<int64_t>(m) * n), batch), TPB, 0, st>>>(m, n, Q, ldq,
-                                                                                          strideQ, diag);
-  return cudaGetLastError();
+  return launch_dependent(set_identity_kernel, dim3(grid_for(static_cast<int64_t>(m) * n), batch), dim3(TPB), 0, st, dim3(1), m, n, Q, ldq, strideQ, diag);
 }
 
 cudaError_t add_diag(int n, double* A, int64_t lda, double d, cudaStream_t st) {
-  add_diag_kernel<<<std::max(1, (n + TPB - 1) / TPB), TPB, 0, st>>>(n, A, lda, d);
-  return cudaGetLastError();
+  return launch_dependent(add_diag_kernel, dim3(std::max(1, (n + TPB - 1) / TPB)), dim3(TPB), 0, st, dim3(1), n, A, lda, d);
 }
 
 }  // namespace zolo

@@ -688,6 +688,8 @@ __global__ void __launch_bounds__(NW * 32, 1) qr_panel_reg_kernel(PanelArgs p) {
 
 __global__ void extract_v_kernel(int m, int w, const double* __restrict__ A, int64_t lda, int64_t strideA,
                                  double* V, int64_t ldv, int64_t strideV, int split, int64_t gap) {
+  dependency_wait();
+  release_dependents();
   const double* Ab = A + blockIdx.y * strideA;
   double* Vb = V + blockIdx.y * strideV;
   const int64_t total = static_cast<int64_t>(m) * w;
@@ -703,6 +705,8 @@ __global__ void extract_v_kernel(int m, int w, const double* __restrict__ A, int
 // QW*QW apart), zero elsewhere: the diagonal of the block reflector's T.
 __global__ void block_t_init_kernel(int jb, const double* __restrict__ T, int64_t strideT, double* TB,
                                     int64_t ldtb, int64_t strideTB) {
+  dependency_wait();
+  release_dependents();
   const double* Tb = T + blockIdx.y * strideT;
   double* Bb = TB + blockIdx.y * strideTB;
   const int total = jb * jb;
@@ -903,16 +907,14 @@ cudaError_t extract_v(int m, int w, const double* A, int64_t lda, int64_t stride
   if (gap < 0 || (gap > 0 && split < w)) return cudaErrorInvalidValue;
   if (!(split > 0 && gap > 0)) split = m;
   int blocks = static_cast<int>(std::min<int64_t>((static_cast<int64_t>(m) * w + 255) / 256, 2048));
-  extract_v_kernel<<<dim3(blocks, batch), 256, 0, st>>>(m, w, A, lda, strideA, V, ldv, strideV, split, gap);
-  return cudaGetLastError();
+  return launch_dependent(extract_v_kernel, dim3(blocks, batch), dim3(256), 0, st, dim3(1), m, w, A, lda, strideA, V, ldv, strideV, split, gap);
 }
 
 cudaError_t block_t_init(int jb, const double* T, int64_t strideT, double* TB, int64_t ldtb, int64_t strideTB,
                          int batch, cudaStream_t st) {
   if (jb <= 0 || batch <= 0) return cudaSuccess;
   const int blocks = (jb * jb + 255) / 256;
-  block_t_init_kernel<<<dim3(blocks, batch), 256, 0, st>>>(jb, T, strideT, TB, ldtb, strideTB);
-  return cudaGetLastError();
+  return launch_dependent(block_t_init_kernel, dim3(blocks, batch), dim3(256), 0, st, dim3(1), jb, T, strideT, TB, ldtb, strideTB);
 }
 
 cudaError_t apply_t(int w, int n, const double* T, int64_t strideT, double* P, int64_t ldp, int64_t strideP,
