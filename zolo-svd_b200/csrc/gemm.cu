@@ -2,10 +2,11 @@
 //
 // tcgen05.mma has no FP64 kind, so the FP64 contractions of the polar
 // iterations (Gram matrix, TRSM updates, Householder trailing updates,
-// Q1*Q2^T) run on DMMA.  General shapes: CTA tile 64x128x16, 8 warps (2 x 4),
-// warp tile 32x32, 3-stage cp.async pipeline, two CTAs per SM (measured 33.1
-// TF/s on a 4096^3 main-loop probe against 30.3 for 128x128 tiles with one CTA
-// per SM; the FP64 tensor pipe saturates at 37.0).  Padded shared-memory
+// Q1*Q2^T) run on DMMA.  General shapes: CTA tile 64x64x16, 4 warps of 32x32, double-buffered
+// cp.async, four CTAs per SM: independent CTAs cover each other's barriers and epilogues, and the
+// small tile leaves less of the last wave idle (4096^3 31.2 TF/s and its lower triangle 29.4, against
+// 31.0 with 64x128 tiles and 27.5 with eight warps on 64x64; V^T C of a 128-column block, 128 x 4096 x
+// 4096 of four, 25 -> 28.7; the FP64 tensor pipe saturates at 37.0).  Padded shared-memory
 // layouts make every fragment load a conflict-free LDS.128 (or LDS.64 for
 // op(B)=B^T).  Products too small for that grid take 32x32 tiles with four warps, and a long K
 // is split over the CTAs of a cluster, which reduce through distributed shared memory
@@ -42,21 +43,21 @@ struct Cfg {
   static constexpr int MI = BM / WM / 16, NJ = BN / WN / 8;
   static constexpr int LDA_N = BM + 2;  // sA[k][m]  (op(A) = A)
   static constexpr int LDB_T = BN + 2;  // sB[k][n]  (op(B) = B^T)
+  static constexpr int SMEM_C = BN * (BM + 2) * 8;  // a tile of C
   __host__ __device__ static constexpr int a_elems(bool ta) { return ta ? BM * LDA_T : BK * LDA_N; }
   __host__ __device__ static constexpr int b_elems(bool tb) { return tb ? BK * LDB_T : BN * LDB_N; }
   __host__ __device__ static constexpr int smem(bool ta, bool tb) { return ST_ * (a_elems(ta) + b_elems(tb)) * 8; }
 };
-using CfgWide = Cfg<64, 128, 2, 4, 3, 2>;     // general: 2 CTAs / SM, warp tile 32x32
+using CfgWide = Cfg<64, 64, 2, 2, 2, 4>;      // general: 4 CTAs / SM of 4 warps, warp tile 32x32
 using CfgSkinnyM = Cfg<32, 64, 1, 8, 4, 3>;    // M <= 32 (V^T W products of the QR updates)
 using CfgSmall = Cfg<64, 64, 2, 4, 2, 3>;      // K <= 64 rank-k updates and N <= 64: 3 CTAs / SM
-using CfgTri = Cfg<64, 64, 2, 4, 3, 3>;        // lower-triangle output (square tiles): 3 CTAs / SM
 using CfgTiny = Cfg<32, 32, 2, 2, 4, 4>;       // products too small to fill the GPU with larger tiles
 
 struct KParams {
   GemmArgs g;
   int tiles_m, tiles_n;
   int splitk;
-  int preload;  // C loaded into the accumulators up front (rank-k updates)
+  int stage_c;  // C copied to shared memory beside the first K tiles (rank-k updates)
 };
 
 template <class C, bool TA, bool TB, bool V16>
@@ -167,45 +168,31 @@ __global__ void __launch_bounds__(C::NT, C::MINB) dgemm_kernel(KParams kp) {
       for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.0;
 
   const int ktiles = (ke > kb) ? (ke - kb + BK - 1) / BK : 0;
-  // Rank-k updates C += alpha A B with |alpha| = 1 (the Householder and TRSM updates) are
-  // bound by streaming C: its tile is loaded into the accumulators before the MMAs, so the
-  // C reads overlap the A/B copies instead of following them.  C is pre-scaled by
-  // beta/alpha (exact for alpha = +-1) and the epilogue then writes alpha * acc.
-  const bool preload = kp.preload;
+  // Rank-k updates C += alpha A B of a short K spend as long on C as on the product: its tile is
+  // copied to shared memory behind the first K tile, so that no thread waits for it.
+  constexpr int LDC_S = BM + 2;
+  double* sC = smem + STAGES * (AE + BE);
+  const bool stage_c = kp.stage_c;
   dependency_wait();
-  if (preload) {
-    const double* Cb = p.C + static_cast<int64_t>(bz) * p.strideC;
-    const double sc = p.beta / p.alpha;
-#pragma unroll
-    for (int i = 0; i < MI; ++i)
-#pragma unroll
-      for (int j = 0; j < NJ; ++j) {
-        const int r = m0 + wm + i * 16 + 2 * g;
-        const int c = n0 + wn + j * 8 + 2 * t;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int cc = c + h;
-          if (cc >= N || r >= M) continue;
-          const double* src = Cb + r + static_cast<int64_t>(cc) * p.ldc;
-          if (V16 && r + 1 < M) {
-            const double2 o = *reinterpret_cast<const double2*>(src);
-            acc[i][j][h] = sc * o.x;
-            acc[i][j][2 + h] = sc * o.y;
-          } else {
-            acc[i][j][h] = sc * src[0];
-            if (r + 1 < M) acc[i][j][2 + h] = sc * src[1];
-          }
-        }
-      }
-  }
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
     if (s < ktiles) load_stage(s, kb + s * BK);
     cp_async_commit();
+    if (s == 0 && stage_c) {
+      const double* Cb = p.C + static_cast<int64_t>(bz) * p.strideC;
+      for (int c = tid; c < BN * (BM / 2); c += NT) {
+        const int n = c / (BM / 2), m = (c % (BM / 2)) * 2;
+        const int gm = m0 + m, gn = n0 + n;
+        const bool ni = gn < N;
+        chunk(sC + n * LDC_S + m, Cb, gm + static_cast<int64_t>(gn) * p.ldc, ni && gm < M, ni && gm + 1 < M);
+      }
+      cp_async_commit();
+    }
   }
 
   for (int kt = 0; kt < ktiles; ++kt) {
-    cp_async_wait<STAGES - 2>();
+    if (kt == 0 && stage_c) cp_async_wait<STAGES - 1>();  // C still on its way
+    else cp_async_wait<STAGES - 2>();
     __syncthreads();
     {
       const int nk = kt + STAGES - 1;
@@ -303,7 +290,8 @@ __global__ void __launch_bounds__(C::NT, C::MINB) dgemm_kernel(KParams kp) {
   double* C_ = p.C + static_cast<int64_t>(bz) * p.strideC;
   const int64_t ldc = p.ldc;
   const double alpha = p.alpha * (p.alpha_vec ? p.alpha_vec[bz] : 1.0);
-  const double beta = preload ? 0.0 : p.beta;
+  const double beta = p.beta;
+  if (stage_c) __syncthreads();
 #pragma unroll
   for (int i = 0; i < MI; ++i)
 #pragma unroll
@@ -321,14 +309,16 @@ __global__ void __launch_bounds__(C::NT, C::MINB) dgemm_kernel(KParams kp) {
         const bool ok1 = (r + 1 < M) && (!p.tri || r + 1 >= cc);
         if (V16 && ok0 && ok1) {
           if (beta != 0.0) {
-            const double2 o = *reinterpret_cast<const double2*>(dst);
+            const double2 o = *reinterpret_cast<const double2*>(
+                stage_c ? sC + wm + i * 16 + 2 * g + (wn + j * 8 + 2 * t + h) * LDC_S : dst);
             v0 += beta * o.x;
             v1 += beta * o.y;
           }
           *reinterpret_cast<double2*>(dst) = make_double2(v0, v1);
         } else {
-          if (ok0) dst[0] = (beta != 0.0) ? v0 + beta * dst[0] : v0;
-          if (ok1) dst[1] = (beta != 0.0) ? v1 + beta * dst[1] : v1;
+          const double* o = stage_c ? sC + wm + i * 16 + 2 * g + (wn + j * 8 + 2 * t + h) * LDC_S : dst;
+          if (ok0) dst[0] = (beta != 0.0) ? v0 + beta * o[0] : v0;
+          if (ok1) dst[1] = (beta != 0.0) ? v1 + beta * o[1] : v1;
         }
       }
     }
@@ -339,10 +329,11 @@ cudaError_t launch_t(const KParams& kp, dim3 grid, cudaStream_t st) {
   static std::atomic<int> attr_set[kMaxDevices];
   const cudaError_t attr = once_per_device(attr_set, [] {
     return cudaFuncSetAttribute(dgemm_kernel<C, TA, TB, V16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                C::smem(TA, TB));
+                                C::smem(TA, TB) + C::SMEM_C);
   });
   if (attr != cudaSuccess) return attr;
-  return launch_dependent(dgemm_kernel<C, TA, TB, V16>, grid, dim3(C::NT), C::smem(TA, TB), st, dim3(1, kp.splitk, 1),
+  return launch_dependent(dgemm_kernel<C, TA, TB, V16>, grid, dim3(C::NT),
+                          C::smem(TA, TB) + (kp.stage_c ? C::SMEM_C : 0), st, dim3(1, kp.splitk, 1),
                           kp);
 }
 
@@ -360,8 +351,8 @@ cudaError_t launch_c(const KParams& kp, dim3 grid, bool v16, cudaStream_t st) {
   return v16 ? launch_v<C, true>(kp, grid, st) : launch_v<C, false>(kp, grid, st);
 }
 
-// tile shape: 0 = 64x128 (general), 1 = 32x64 (M <= 32), 2 = 64x64 (K <= 64 or N <= 64),
-// 3 = 64x64 with 3 stages (lower-triangle output), 4 = 32x32 (too small to fill the GPU)
+// tile shape: 0 = 64x64 with four warps (general), 1 = 32x64 (M <= 32), 2 = 64x64 with eight warps
+// (K <= 64 or N <= 64, and short-K updates), 4 = 32x32 (too small to fill the GPU)
 int pick_cfg(const GemmArgs& a) {
   // Products that leave SMs idle with 64 x 64 tiles (FP64 DMMA runs at 64 FMA a clock and SM, so a
   // tile of K = 64 alone takes 2.1 us): 32 x 32 tiles spread them wider.  Measured 64 x 64 against
@@ -372,12 +363,12 @@ int pick_cfg(const GemmArgs& a) {
   const int64_t tiles64 = (a.tri ? t64 * (t64 + 1) / 2 : t64 * u64) * a.batch;
   const double work = static_cast<double>(a.M) * a.N * a.K * a.batch * (a.tri ? 0.5 : 1.0);
   if (tiles64 < num_sms() && work <= 1.4e8) return 4;
-  if (a.tri) return 3;
+  if (a.tri) return 0;
   if (a.M <= 32) return 1;
   if (a.K <= 64 || a.N <= 64) return 2;
   // C += A B updates with K <= 256 (the 128-column block reflector updates of the QR):
-  // 64 x 64 tiles, three CTAs per SM, C loaded up front (21.7 TF/s against 18.7 for
-  // 64 x 128 tiles at M = 16384, N = 4096, K = 128)
+  // eight warps, three CTAs per SM, C staged in shared memory (8192 x 8064 x 128: 25.9 TF/s, 22.5 when C
+  // was loaded into the accumulators first, 24.7 with four warps)
   if (a.K <= 256 && !a.transA && a.beta != 0.0) return 2;
   return 0;
 }
@@ -395,15 +386,36 @@ void tile_dims(int cfg, int* bm, int* bn, int* per_sm) {
     *bm = CfgSmall::BM;
     *bn = CfgSmall::BN;
     *per_sm = CfgSmall::MINB;
-  } else if (cfg == 3) {
-    *bm = CfgTri::BM;
-    *bn = CfgTri::BN;
-    *per_sm = CfgTri::MINB;
   } else {
     *bm = CfgWide::BM;
     *bn = CfgWide::BN;
     *per_sm = CfgWide::MINB;
   }
+}
+
+// Slices of K for the general tiles, 4 CTAs an SM: the time in K tiles of one CTA per SM at the full
+// rate is (kt / s + 2) for every CTA of a slot, and a last wave of 1, 2, 3 or 4 CTAs an SM takes as
+// long as 1.75, 2.5, 3.2 or 4 of them (28 % of the FP64 tensor rate a CTA alone reaches, 80 % three).
+// Powers of two: clusters of 3, 5 or 7 leave SMs of a GPC idle (with 64 x 128 tiles, 128 x 1024 x 3072
+// of six ran at 18.3, 18.4 and 24.3 TF/s in 2, 3 and 4 slices).  Measured against one slice:
+// 128 x 8064 x 8192 20.1 -> 25.7, 128 x 2048 x 2048 of six 24.6 -> 27.6, 1024^3 19.7 -> 22.5, lower
+// triangle of 2048^3 25.0 -> 27.6 TF/s; 2048^3 stays whole (29.7).
+int split_general(int64_t ctas, int kt, int sms) {
+  static const double last[5] = {0.0, 1.75, 2.5, 3.2, 4.0};
+  constexpr int per_sm = CfgWide::MINB;
+  static_assert(per_sm == 4, "the last wave's times are for four CTAs an SM");
+  int best = 1;
+  double best_t = 1e300;
+  for (int s = 1; s <= 8 && s <= kt; s *= 2) {
+    const int64_t n = ctas * s, wave = static_cast<int64_t>(sms) * per_sm;
+    const int64_t rest = n % wave;
+    const double t = ((kt + s - 1) / s + 2) * (static_cast<double>(n / wave) * per_sm + last[(rest + sms - 1) / sms]);
+    if (t < best_t * (1.0 - 1e-9)) {
+      best_t = t;
+      best = s;
+    }
+  }
+  return best;
 }
 
 // Split K only when the tile grid cannot fill the GPU; pick the split (the CTAs of one portable
@@ -418,8 +430,9 @@ int choose_splitk(const GemmArgs& a, int sms) {
   const int64_t tiles = a.tri ? static_cast<int64_t>(tm) * (tm + 1) / 2 : static_cast<int64_t>(tm) * tn;
   const int64_t ctas = tiles * a.batch;
   const int64_t wave = static_cast<int64_t>(sms) * per_sm;
-  if (ctas >= wave) return 1;
   const int kt = (a.K + BK - 1) / BK;
+  if (cfg == 0) return split_general(ctas, kt, sms);
+  if (ctas >= wave) return 1;
   const int smax = std::min(8, kt / (cfg == 4 ? 4 : 8));
   if (smax < 2) return 1;
   int best = 1;
@@ -475,7 +488,7 @@ cudaError_t dgemm(GemmArgs a, cudaStream_t st) {
   kp.tiles_m = (a.M + BM - 1) / BM;
   kp.tiles_n = (a.N + BN - 1) / BN;
   kp.splitk = choose_splitk(a, sms);
-  kp.preload = (kp.splitk <= 1 && a.beta != 0.0 && !a.tri && !a.kto_m && !a.alpha_vec &&
+  kp.stage_c = (kp.splitk <= 1 && a.beta != 0.0 && !a.tri && !a.kto_m && !a.alpha_vec &&
                  (a.alpha == 1.0 || a.alpha == -1.0) && (a.K <= 64 || (cfg == 2 && a.K <= 256)))
                    ? 1
                    : 0;
@@ -485,7 +498,6 @@ cudaError_t dgemm(GemmArgs a, cudaStream_t st) {
   dim3 grid(static_cast<unsigned>(tiles), kp.splitk, a.batch);
   const cudaError_t e = cfg == 1   ? launch_c<CfgSkinnyM>(kp, grid, v16, st)
                         : cfg == 2 ? launch_c<CfgSmall>(kp, grid, v16, st)
-                        : cfg == 3 ? launch_c<CfgTri>(kp, grid, v16, st)
                         : cfg == 4 ? launch_c<CfgTiny>(kp, grid, v16, st)
                                    : launch_c<CfgWide>(kp, grid, v16, st);
   return e;
