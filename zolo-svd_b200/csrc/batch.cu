@@ -36,15 +36,12 @@ __device__ double block_sum_b(double v, double* sh) {
 __global__ void pack_kernel(const BatchMember* mem, int MB, int NB, double* P, int64_t ldp, int64_t sp) {
   const BatchMember d = mem[blockIdx.y];
   double* Pb = P + blockIdx.y * sp;
-  const int64_t total = static_cast<int64_t>(MB) * NB;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % MB), j = static_cast<int>(e / MB);
+  for_entries(MB, NB, [&](int i, int j) {
     double v;
     if (j < d.n) v = (i < d.m) ? d.A[i + static_cast<int64_t>(j) * d.lda] : 0.0;
     else v = (i == d.m + (j - d.n)) ? d.tau : 0.0;
     Pb[i + static_cast<int64_t>(j) * ldp] = v;
-  }
+  });
 }
 
 // Q_b = Q'(b)[0:m, 0:n], H_b = H'(b)[0:n, 0:n]
@@ -53,19 +50,13 @@ __global__ void unpack_kernel(const BatchMember* mem, const double* Q, int64_t l
   const BatchMember d = mem[blockIdx.y];
   const double* Qb = Q + blockIdx.y * sq;
   const double* Hb = H ? H + blockIdx.y * sh : nullptr;
-  const int64_t tq = static_cast<int64_t>(d.m) * d.n;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < tq;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % d.m), j = static_cast<int>(e / d.m);
+  for_entries(d.m, d.n, [&](int i, int j) {
     d.Q[i + static_cast<int64_t>(j) * d.ldq] = Qb[i + static_cast<int64_t>(j) * ldq];
-  }
+  });
   if (Hb && d.H) {
-    const int64_t th = static_cast<int64_t>(d.n) * d.n;
-    for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < th;
-         e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-      const int i = static_cast<int>(e % d.n), j = static_cast<int>(e / d.n);
+    for_entries(d.n, d.n, [&](int i, int j) {
       d.H[i + static_cast<int64_t>(j) * d.ldh] = Hb[i + static_cast<int64_t>(j) * ldh];
-    }
+    });
   }
 }
 
@@ -73,14 +64,11 @@ __global__ void unpack_kernel(const BatchMember* mem, const double* Q, int64_t l
 __global__ void frob2_batch_kernel(int m, int n, const double* X, int64_t ldx, int64_t sx, double* partial) {
   __shared__ double sh[TPB / 32];
   const double* Xb = X + blockIdx.y * sx;
-  const int64_t total = static_cast<int64_t>(m) * n;
   double s = 0.0;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % m), j = static_cast<int>(e / m);
+  for_entries(m, n, [&](int i, int j) {
     const double x = Xb[i + static_cast<int64_t>(j) * ldx];
     s += x * x;
-  }
+  });
   s = block_sum_b<TPB>(s, sh);
   if (threadIdx.x == 0) partial[blockIdx.y * gridDim.x + blockIdx.x] = s;
 }
@@ -94,13 +82,15 @@ __global__ void reduce_rows_kernel(const double* partial, int nb, double* out) {
   if (threadIdx.x == 0) out[blockIdx.x] = s;
 }
 
-// out[b] = max_j sum_i |X_b(i, j)|  (one CTA per member, a warp per column)
+// out[b] = max(out[b], max_j sum_i |X_b(i, j)|), a warp per column; out starts at zero (the maximum of
+// non-negative values by their bits, the same in any order).  One CTA a member was 540 us for a
+// bucket of the 512-matrix batch, on a few SMs.
 __global__ void norm1_batch_kernel(int m, int n, const double* X, int64_t ldx, int64_t sx, double* out) {
   __shared__ double sh[TPB / 32];
-  const double* Xb = X + blockIdx.x * sx;
+  const double* Xb = X + blockIdx.y * sx;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double best = 0.0;
-  for (int j = warp; j < n; j += TPB / 32) {
+  for (int j = blockIdx.x * (TPB / 32) + warp; j < n; j += gridDim.x * (TPB / 32)) {
     double s = 0.0;
     for (int i = lane; i < m; i += 32) s += fabs(Xb[i + static_cast<int64_t>(j) * ldx]);
     s = warp_sum(s);
@@ -111,7 +101,8 @@ __global__ void norm1_batch_kernel(int m, int n, const double* X, int64_t ldx, i
   if (threadIdx.x == 0) {
     double b = 0.0;
     for (int w = 0; w < TPB / 32; ++w) b = fmax(b, sh[w]);
-    out[blockIdx.x] = b;
+    atomicMax(reinterpret_cast<unsigned long long*>(out + blockIdx.y),
+              static_cast<unsigned long long>(__double_as_longlong(b)));
   }
 }
 
@@ -119,12 +110,9 @@ __global__ void norm1_batch_kernel(int m, int n, const double* X, int64_t ldx, i
 __global__ void scale_batch_kernel(int m, int n, double* X, int64_t ldx, int64_t sx, const double* s) {
   double* Xb = X + blockIdx.y * sx;
   const double f = s[blockIdx.y];
-  const int64_t total = static_cast<int64_t>(m) * n;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % m), j = static_cast<int>(e / m);
+  for_entries(m, n, [&](int i, int j) {
     Xb[i + static_cast<int64_t>(j) * ldx] *= f;
-  }
+  });
 }
 
 // X_b <- cx_b X_b + cz_b Z_b, partial[b * nb + block] = sum (X_new - X_old)^2
@@ -134,17 +122,14 @@ __global__ void combine_batch_kernel(int m, int n, double* X, int64_t ldx, int64
   double* Xb = X + blockIdx.y * sx;
   const double* Zb = Z + blockIdx.y * sz;
   const double a = cx[blockIdx.y], c = cz[blockIdx.y];
-  const int64_t total = static_cast<int64_t>(m) * n;
   double s = 0.0;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % m), j = static_cast<int>(e / m);
+  for_entries(m, n, [&](int i, int j) {
     const double x = Xb[i + static_cast<int64_t>(j) * ldx];
     const double xn = (c == 0.0) ? x : a * x + c * Zb[i + static_cast<int64_t>(j) * ldz];
     const double d = xn - x;
     s += d * d;
     Xb[i + static_cast<int64_t>(j) * ldx] = xn;
-  }
+  });
   s = block_sum_b<TPB>(s, sh);
   if (threadIdx.x == 0) partial[blockIdx.y * gridDim.x + blockIdx.x] = s;
 }
@@ -178,16 +163,13 @@ __global__ void add_diag_batch_kernel(int n, double* G, int64_t ldg, int64_t sg,
 // B_b <- (B_b + B_b^T)/2
 __global__ void symmetrize_batch_kernel(int n, double* B, int64_t ldb, int64_t sb) {
   double* Bb = B + blockIdx.y * sb;
-  const int64_t total = static_cast<int64_t>(n) * n;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % n), j = static_cast<int>(e / n);
-    if (i <= j) continue;
+  for_entries(n, n, [&](int i, int j) {
+    if (i <= j) return;
     const double x = Bb[i + static_cast<int64_t>(j) * ldb], y = Bb[j + static_cast<int64_t>(i) * ldb];
     const double h = 0.5 * y + 0.5 * x;
     Bb[i + static_cast<int64_t>(j) * ldb] = h;
     Bb[j + static_cast<int64_t>(i) * ldb] = h;
-  }
+  });
 }
 
 // B_b = A_b^T  (A m x n)
@@ -241,7 +223,10 @@ cudaError_t batch_frob2(int m, int n, const double* X, int64_t ldx, int64_t sx, 
 cudaError_t batch_norm1(int m, int n, const double* X, int64_t ldx, int64_t sx, int batch, double* out,
                         cudaStream_t st) {
   if (batch <= 0) return cudaSuccess;
-  norm1_batch_kernel<<<batch, TPB, 0, st>>>(m, n, X, ldx, sx, out);
+  const cudaError_t e = cudaMemsetAsync(out, 0, sizeof(double) * batch, st);
+  if (e != cudaSuccess) return e;
+  const int nb = std::max(1, std::min((n + TPB / 32 - 1) / (TPB / 32), 8 * num_sms() / batch));
+  norm1_batch_kernel<<<dim3(nb, batch), TPB, 0, st>>>(m, n, X, ldx, sx, out);
   return cudaGetLastError();
 }
 

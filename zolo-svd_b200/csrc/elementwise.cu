@@ -27,14 +27,11 @@ __global__ void scale_copy_kernel(int m, int n, double s, const double* __restri
   const int b = blockIdx.y;
   const double* S = src + b * strideS;
   double* D = dst + b * strideD;
-  const int64_t total = static_cast<int64_t>(m) * n;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % m), j = static_cast<int>(e / m);
+  for_entries(m, n, [&](int i, int j) {
     double v = s * S[i + j * lds];
     if (i == j) v += diag_add;
     D[i + j * ldd] = v;
-  }
+  });
 }
 
 __global__ void form_stack_kernel(int m, int mpad, int n, const double* __restrict__ X, int64_t ldx, double* W,
@@ -47,15 +44,12 @@ __global__ void form_stack_kernel(int m, int mpad, int n, const double* __restri
   double* Wb = W + b * strideW;
   const double s = s_vec ? s_vec[b] : s_scalar;
   const int rows = mpad + n;
-  const int64_t total = static_cast<int64_t>(rows) * n;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % rows), j = static_cast<int>(e / rows);
+  for_entries(rows, n, [&](int i, int j) {
     double v;
     if (i < m) v = (x_upper && i > j) ? 0.0 : X[i + j * ldx];
     else v = (i - mpad == j) ? s : 0.0;
     Wb[i + j * ldw] = v;
-  }
+  });
 }
 
 __global__ void shift_lower_kernel(int n, const double* __restrict__ G, int64_t ldg, double* W,
@@ -65,15 +59,12 @@ __global__ void shift_lower_kernel(int n, const double* __restrict__ G, int64_t 
   const int b = blockIdx.y;
   double* Wb = W + b * strideW;
   const double c = c_vec[b];
-  const int64_t total = static_cast<int64_t>(n) * n;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % n), j = static_cast<int>(e / n);
-    if (i < j) continue;
+  for_entries(n, n, [&](int i, int j) {
+    if (i < j) return;
     double v = G[i + j * ldg];
     if (i == j) v += c;
     Wb[i + j * ldw] = v;
-  }
+  });
 }
 
 template <int BS>
@@ -94,14 +85,11 @@ __global__ void frob2_kernel(int m, int n, const double* __restrict__ X, int64_t
   dependency_wait();
   release_dependents();
   __shared__ double sh[TPB / 32];
-  const int64_t total = static_cast<int64_t>(m) * n;
   double s = 0.0;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % m), j = static_cast<int>(e / m);
+  for_entries(m, n, [&](int i, int j) {
     const double v = X[i + j * ldx];
     s += v * v;
-  }
+  });
   s = block_sum<TPB>(s, sh);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
@@ -150,11 +138,8 @@ __global__ void combine_kernel(int m, int n, double* X, int64_t ldx, const doubl
   dependency_wait();
   release_dependents();
   __shared__ double sh[TPB / 32];
-  const int64_t total = static_cast<int64_t>(m) * n;
   double s = 0.0;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % m), j = static_cast<int>(e / m);
+  for_entries(m, n, [&](int i, int j) {
     const double x = X[i + j * ldx];
     double z = 0.0;
     if (cz_vec) {
@@ -167,7 +152,7 @@ __global__ void combine_kernel(int m, int n, double* X, int64_t ldx, const doubl
     const double d = x - xn;
     s += d * d;
     X[i + j * ldx] = xn;
-  }
+  });
   s = block_sum<TPB>(s, sh);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
@@ -175,16 +160,13 @@ __global__ void combine_kernel(int m, int n, double* X, int64_t ldx, const doubl
 __global__ void symmetrize_kernel(int n, double* B, int64_t ldb) {
   dependency_wait();
   release_dependents();
-  const int64_t total = static_cast<int64_t>(n) * n;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % n), j = static_cast<int>(e / n);
-    if (i <= j) continue;  // each pair once, by the lower element
+  for_entries(n, n, [&](int i, int j) {
+    if (i <= j) return;  // each pair once, by the lower element
     const double a = B[i + j * ldb], b = B[j + i * ldb];
     const double h = 0.5 * b + 0.5 * a;
     B[i + j * ldb] = h;
     B[j + i * ldb] = h;
-  }
+  });
 }
 
 __global__ void transpose_kernel(int m, int n, const double* __restrict__ A, int64_t lda, double* B,
@@ -211,20 +193,17 @@ __global__ void ns_prepare_kernel(int n, double* G, int64_t ldg, int write, doub
   dependency_wait();
   release_dependents();
   __shared__ double sh[TPB / 32];
-  const int64_t total = static_cast<int64_t>(n) * n;
   double s = 0.0;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % n), j = static_cast<int>(e / n);
-    if (i < j) continue;
+  for_entries(n, n, [&](int i, int j) {
+    if (i < j) return;
     const double g = G[i + j * ldg];
     const double d = (i == j) ? g - 1.0 : g;
     s += (i == j) ? d * d : 2.0 * d * d;
-    if (!write) continue;
+    if (!write) return;
     const double v = (i == j) ? 1.5 - 0.5 * g : -0.5 * g;
     G[i + j * ldg] = v;
     if (i != j) G[j + i * ldg] = v;
-  }
+  });
   s = block_sum<TPB>(s, sh);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
@@ -233,36 +212,27 @@ __global__ void ns_prepare_kernel(int n, double* G, int64_t ldg, int write, doub
 __global__ void mirror_lower_kernel(int n, double* B, int64_t ldb) {
   dependency_wait();
   release_dependents();
-  const int64_t total = static_cast<int64_t>(n) * n;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % n), j = static_cast<int>(e / n);
+  for_entries(n, n, [&](int i, int j) {
     if (i > j) B[j + static_cast<int64_t>(i) * ldb] = B[i + static_cast<int64_t>(j) * ldb];
-  }
+  });
 }
 
 __global__ void copy_upper_kernel(int n, const double* __restrict__ A, int64_t lda, double scale, double* B,
                                   int64_t ldb) {
   dependency_wait();
   release_dependents();
-  const int64_t total = static_cast<int64_t>(n) * n;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % n), j = static_cast<int>(e / n);
+  for_entries(n, n, [&](int i, int j) {
     B[i + static_cast<int64_t>(j) * ldb] = (i <= j) ? scale * A[i + static_cast<int64_t>(j) * lda] : 0.0;
-  }
+  });
 }
 
 __global__ void set_identity_kernel(int m, int n, double* Q, int64_t ldq, int64_t strideQ, double diag) {
   dependency_wait();
   release_dependents();
   double* Qb = Q + blockIdx.y * strideQ;
-  const int64_t total = static_cast<int64_t>(m) * n;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % m), j = static_cast<int>(e / m);
+  for_entries(m, n, [&](int i, int j) {
     Qb[i + j * ldq] = (i == j) ? diag : 0.0;
-  }
+  });
 }
 
 __global__ void add_diag_kernel(int n, double* A, int64_t lda, double d) {
@@ -281,13 +251,10 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
 }
 
 __global__ void fill_random_kernel(int m, int n, double* X, int64_t ldx, uint64_t seed) {
-  const int64_t total = static_cast<int64_t>(m) * n;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % m), j = static_cast<int>(e / m);
-    const uint64_t r = mix64(seed * 0x100000001B3ull + static_cast<uint64_t>(e));
+  for_entries(m, n, [&](int i, int j) {
+    const uint64_t r = mix64(seed * 0x100000001B3ull + static_cast<uint64_t>(i + static_cast<int64_t>(j) * m));
     X[i + j * ldx] = 2.0 * (static_cast<double>(r >> 11) * (1.0 / 9007199254740992.0)) - 1.0;
-  }
+  });
 }
 
 __global__ void trace_kernel(int n, const double* A, int64_t lda, double* out) {
@@ -300,12 +267,9 @@ __global__ void trace_kernel(int n, const double* A, int64_t lda, double* out) {
 
 __global__ void gather_columns_kernel(int m, int n, const double* __restrict__ A, int64_t lda, const int* perm,
                                       double* B, int64_t ldb) {
-  const int64_t total = static_cast<int64_t>(m) * n;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % m), j = static_cast<int>(e / m);
+  for_entries(m, n, [&](int i, int j) {
     B[i + j * ldb] = A[i + static_cast<int64_t>(perm[j]) * lda];
-  }
+  });
 }
 
 __global__ void get_diag_kernel(int n, const double* A, int64_t lda, double* d) {

@@ -692,13 +692,10 @@ __global__ void extract_v_kernel(int m, int w, const double* __restrict__ A, int
   release_dependents();
   const double* Ab = A + blockIdx.y * strideA;
   double* Vb = V + blockIdx.y * strideV;
-  const int64_t total = static_cast<int64_t>(m) * w;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(e % m), j = static_cast<int>(e / m);
+  for_entries(m, w, [&](int i, int j) {
     double v = (i > j) ? Ab[i + (i >= split ? gap : 0) + j * lda] : (i == j ? 1.0 : 0.0);
     Vb[i + j * ldv] = v;
-  }
+  });
 }
 
 // TB (jb x jb) <- the block diagonal of consecutive panels' T factors (QW x QW each, ld QW,
