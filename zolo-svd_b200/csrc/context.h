@@ -208,6 +208,30 @@ struct EventTimer {
   }
 };
 
+// Times of a stream's phases without a wait at each end: events recorded as the work is queued,
+// read once it has run.
+struct EventMarks {
+  std::vector<cudaEvent_t> ev;
+  int mark(cudaStream_t st) {
+    cudaEvent_t e = nullptr;
+    ck(cudaEventCreate(&e));
+    ev.push_back(e);
+    ck(cudaEventRecord(e, st));
+    return static_cast<int>(ev.size()) - 1;
+  }
+  double ms(int a, int b) const {
+    float v = 0.f;
+    ck(cudaEventElapsedTime(&v, ev[a], ev[b]));
+    return v;
+  }
+  EventMarks() = default;
+  EventMarks(const EventMarks&) = delete;
+  EventMarks& operator=(const EventMarks&) = delete;
+  ~EventMarks() {
+    for (auto e : ev) cudaEventDestroy(e);
+  }
+};
+
 // Routes the large products of gemm() to the INT8-emulated GEMM while in scope (when the
 // handle's mixed form is on), and restores the previous routing on exit.
 struct OzScope {

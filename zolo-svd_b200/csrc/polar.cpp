@@ -330,21 +330,14 @@ int bounds(Context& c, int m, int n, double sigma, const double* dA, int64_t lda
   ck(scale_copy(m, n, 1.0, dA, lda, 0, X, ldx, 0, 1, -sigma, c.stream()));
   ck(frob2(m, n, X, ldx, part, scal, c.stream()));
   c.stats.launches += 3;
-  const double a = std::sqrt(d2h(c, scal));
-  *alpha = a;
-  if (alpha_fro) *alpha_fro = a;
-  if (!(a > 0.0) || !std::isfinite(a)) {
-    *beta = 0.0;
-    return 1;
-  }
-  ck(scale_copy(m, n, 1.0 / a, X, ldx, 0, X, ldx, 0, 1, 0.0, c.stream()));
+  // scaled by 1 / ||A||_F on the device: the norms come back together at the end (each read-back
+  // left the GPU idle for 30 us); a zero or non-finite norm is found there
+  ck(scale_by_norm(m, n, scal, X, ldx, c.stream()));
   c.stats.launches++;
-  double temp_beta = 1.0;
   if (mode == BOUNDS_PQDWHFACS) {
     double* colsum = c.buf("bnd_colsum", n);
     ck(norm1(m, n, X, ldx, colsum, scal + 1, c.stream()));
     c.stats.launches += 2;
-    temp_beta = d2h(c, scal + 1);
   }
   // R of X = QR (unstructured Householder), then R^{-T} = (R^T)^{-1} by the blocked triangular
   // inverse and R^{-1} as its transpose for ||R^{-1}||_1 and ||R^{-1}||_F
@@ -363,8 +356,17 @@ int bounds(Context& c, int m, int n, double sigma, const double* dA, int64_t lda
   ck(norm1(n, n, Ri, ldn, colsum, scal + 2, c.stream()));
   ck(frob2(n, n, Ri, ldn, part, scal + 3, c.stream()));
   c.stats.launches += 4;
-  const double inv1 = d2h(c, scal + 2);
-  const double fr = d2h(c, scal + 3);
+  double nv[4];
+  ck(cudaMemcpyAsync(nv, scal, sizeof(nv), cudaMemcpyDeviceToHost, c.stream()));
+  ck(cudaStreamSynchronize(c.stream()));
+  const double a = std::sqrt(nv[0]);
+  *alpha = a;
+  if (alpha_fro) *alpha_fro = a;
+  if (!(a > 0.0) || !std::isfinite(a)) {
+    *beta = 0.0;
+    return 1;
+  }
+  const double temp_beta = mode == BOUNDS_PQDWHFACS ? nv[1] : 1.0, inv1 = nv[2], fr = nv[3];
   c.stats.flops += 4.0 / 3.0 * static_cast<double>(n) * n * n + 2.0 * m * static_cast<double>(n) * n;
   if (!std::isfinite(fr) || !std::isfinite(inv1) || !(inv1 > 0.0)) {
     *beta = 0.0;
@@ -387,7 +389,8 @@ int qdwh(Context& c, int m, int n, const double* dA, int64_t lda, double* dQ, in
   if (m < n) return -1;
   if (m == 0 || n == 0) return 0;
   c.stats = Stats{};
-  EventTimer total(c.stream());
+  EventMarks marks;
+  const int t_start = marks.mark(c.stream());
   // internal copies with an even leading dimension (16-byte aligned GEMM tiles)
   const int64_t ldx = even(m);
   double* Ain = c.buf("Ain", static_cast<size_t>(ldx) * n);
@@ -396,9 +399,11 @@ int qdwh(Context& c, int m, int n, const double* dA, int64_t lda, double* dQ, in
   c.stats.launches++;
   double alpha = 0, beta = 0;
   {
-    EventTimer tb(c.stream());
+    const int t_bounds = marks.mark(c.stream());
     const int info = bounds(c, m, n, o.sigma, Ain, ldx, o.bounds, &alpha, &beta);
-    c.stats.ms_bounds = tb.stop();
+    const int t_done = marks.mark(c.stream());
+    ck(cudaEventSynchronize(marks.ev[t_done]));
+    c.stats.ms_bounds = marks.ms(t_bounds, t_done);
     c.stats.alpha = alpha;
     c.stats.beta = beta;
     if (info != 0) {
@@ -406,9 +411,6 @@ int qdwh(Context& c, int m, int n, const double* dA, int64_t lda, double* dQ, in
       return info;
     }
   }
-  ck(scale_copy(m, n, 1.0, Ain, ldx, 0, X, ldx, 0, 1, -o.sigma, c.stream()));
-  ck(scale_copy(m, n, 1.0 / alpha, X, ldx, 0, X, ldx, 0, 1, 0.0, c.stream()));
-  c.stats.launches += 2;
 
   const double eps = eps_precision();
   const double tol1 = 10.0 * eps / 2.0;
@@ -427,74 +429,124 @@ int qdwh(Context& c, int m, int n, const double* dA, int64_t lda, double* dQ, in
   double* part = c.dpartial();
   const bool left = (o.left_solve || o.sym == 'S' || o.sym == 's') && m == n;
 
-  EventTimer ti(c.stream());
-  double lowk = beta, err = 1.0, err2 = std::fabs(1.0 - lowk);
-  int it = 0;
-  while ((it == 0 || err > tol2 || err2 > tol1) && (o.maxit < 0 || it <= o.maxit) && it < 100) {
-    EventTimer tstep(c.stream());
-    double ak, bk, ckk, lnext;
-    qdwh_weights(lowk, &ak, &bk, &ckk, &lnext);
-    lowk = lnext;
-    double akk, bkk;
-    bool use_qr = ckk > 100.0;
-    if (!use_qr) {
-      OzScope mixed_ch(c, c.zolo_mixed >= 1);  // the mixed form's products of this Cholesky step
-      gemm(c, 1, 0, n, n, m, ckk, Mat{X, ldx, 0}, Mat{X, ldx, 0}, 0.0, G, 1, nullptr, 1, 0);
-      ck(add_diag(n, G.p, G.ld, 1.0, c.stream()));
-      ck(cudaMemsetAsync(dinfo, 0, sizeof(int), c.stream()));
-      c.stats.launches += 2;
-      potrf_inv(c, n, G, Y, 1, dinfo);
-      const int pinfo = injected_info(c, it, read_info(c, dinfo, 1));
-      if (pinfo != 0) {
-        // not numerically SPD: redo this step with the QR form (the reference ignores PDPOSV's INFO)
-        if (c.stats.info == 0) c.stats.info = pinfo;
-        use_qr = true;
-      } else {
-        spd_solve(c, m, n, X, ldx, Y, Z, 1, left);
-        akk = ak - bk / ckk;
-        bkk = bk / ckk;
-        c.stats.chol_iterations++;
-        if (it < 16) c.stats.branch[it] = 2;
-        c.stats.flops += 2.0 * m * static_cast<double>(n) * n + static_cast<double>(n) * n * n / 3.0 +
-                         static_cast<double>(m) * n * n;
+  // The loop ends on ||X_{k+1} - X_k||_F only once L has converged, and L follows from L_0 alone: up
+  // to there no step waits for the host.  Errors and Cholesky INFO stay on the device, a slot a
+  // step, and come back together; a failed factorization is found then and the loop runs again
+  // from X_0, reading INFO before each solve.  (One read-back and one wait a step left the GPU idle
+  // for 35 us each: QDWH n = 96 0.98 -> 0.77 ms.)
+  constexpr int kSlots = 16;
+  double* errs = scal + 32;
+  const Stats stats0 = c.stats;
+  const int t_loop = marks.mark(c.stream());
+  int it = 0, t_end = t_loop;
+  double err = 1.0;
+  auto iterate = [&](bool careful) -> bool {
+    std::vector<int> t_step{marks.mark(c.stream())};
+    ck(scale_copy(m, n, 1.0, Ain, ldx, 0, X, ldx, 0, 1, -o.sigma, c.stream()));
+    ck(scale_copy(m, n, 1.0 / alpha, X, ldx, 0, X, ldx, 0, 1, 0.0, c.stream()));
+    ck(cudaMemsetAsync(dinfo, 0, sizeof(int) * kSlots, c.stream()));
+    c.stats.launches += 3;
+    double herr[kSlots];
+    int hinfo[kSlots], have = 0;  // steps read back
+    // errors and INFO of the steps so far; false when a factorization failed
+    auto read_back = [&]() {
+      ck(cudaMemcpyAsync(herr, errs, sizeof(herr), cudaMemcpyDeviceToHost, c.stream()));
+      ck(cudaMemcpyAsync(hinfo, dinfo, sizeof(hinfo), cudaMemcpyDeviceToHost, c.stream()));
+      ck(cudaStreamSynchronize(c.stream()));
+      have = it;
+      for (int k = 0; k < std::min(it, kSlots); ++k) {
+        if (!careful && c.stats.branch[k] == 2 && injected_info(c, k, hinfo[k]) != 0) return false;
+        c.stats.err[k] = std::sqrt(herr[k]);
       }
+      return true;
+    };
+    double lowk = beta, err2 = std::fabs(1.0 - lowk);
+    it = 0;
+    err = 1.0;
+    while ((o.maxit < 0 || it <= o.maxit) && it < 100) {
+      const int slot = std::min(it, kSlots - 1);
+      if (it > 0 && (careful || err2 <= tol1)) {
+        if (!careful && !read_back()) return false;
+        err = careful ? std::sqrt(d2h(c, errs + std::min(it - 1, kSlots - 1))) : c.stats.err[it - 1];
+        if (!(err > tol2 || err2 > tol1)) break;
+      }
+      if (!careful && it == kSlots) return false;  // no slot for another step
+      double ak, bk, ckk, lnext;
+      qdwh_weights(lowk, &ak, &bk, &ckk, &lnext);
+      lowk = lnext;
+      double akk, bkk;
+      bool use_qr = ckk > 100.0;
+      if (!use_qr) {
+        OzScope mixed_ch(c, c.zolo_mixed >= 1);  // the mixed form's products of this Cholesky step
+        gemm(c, 1, 0, n, n, m, ckk, Mat{X, ldx, 0}, Mat{X, ldx, 0}, 0.0, G, 1, nullptr, 1, 0);
+        ck(add_diag(n, G.p, G.ld, 1.0, c.stream()));
+        c.stats.launches++;
+        if (careful) {
+          ck(cudaMemsetAsync(dinfo + slot, 0, sizeof(int), c.stream()));
+          c.stats.launches++;
+        }
+        potrf_inv(c, n, G, Y, 1, dinfo + slot);
+        const int pinfo = careful ? injected_info(c, it, read_info(c, dinfo + slot, 1)) : 0;
+        if (pinfo != 0) {
+          // not numerically SPD: redo this step with the QR form (the reference ignores PDPOSV's INFO)
+          if (c.stats.info == 0) c.stats.info = pinfo;
+          use_qr = true;
+        } else {
+          spd_solve(c, m, n, X, ldx, Y, Z, 1, left);
+          akk = ak - bk / ckk;
+          bkk = bk / ckk;
+          c.stats.chol_iterations++;
+          if (it < 16) c.stats.branch[it] = 2;
+          c.stats.flops += 2.0 * m * static_cast<double>(n) * n + static_cast<double>(n) * n * n / 3.0 +
+                           static_cast<double>(m) * n * n;
+        }
+      }
+      if (use_qr) {
+        const double sck = std::sqrt(ckk);
+        ck(form_stack(m, mp, n, X, ldx, W.p, W.ld, 0, nullptr, 1.0 / sck, 1, c.stream()));
+        c.stats.launches++;
+        geqrf(c, mp + n, n, mp, W, tau, T, 1);
+        orgqr(c, mp + n, n, mp, W, T, Qf, 1);
+        q1q2t(c, m, mp, n, Qf, Z, 1);
+        akk = (ak - bk / ckk) / sck;
+        bkk = bk / ckk;
+        c.stats.qr_iterations++;
+        if (it < 16) c.stats.branch[it] = 1;
+        c.stats.flops += 4.0 * m * static_cast<double>(n) * n + static_cast<double>(n) * n * n;
+      }
+      ck(combine_update(m, n, X, ldx, Z.p, Z.ld, 0, 1, bkk, akk, nullptr, part, errs + slot, c.stream()));
+      c.stats.launches += 2;
+      if (it < 16) c.stats.con[it] = ckk;
+      t_step.push_back(marks.mark(c.stream()));
+      ++it;
+      err2 = std::fabs(1.0 - lowk);
     }
-    if (use_qr) {
-      const double sck = std::sqrt(ckk);
-      ck(form_stack(m, mp, n, X, ldx, W.p, W.ld, 0, nullptr, 1.0 / sck, 1, c.stream()));
-      c.stats.launches++;
-      geqrf(c, mp + n, n, mp, W, tau, T, 1);
-      orgqr(c, mp + n, n, mp, W, T, Qf, 1);
-      q1q2t(c, m, mp, n, Qf, Z, 1);
-      akk = (ak - bk / ckk) / sck;
-      bkk = bk / ckk;
-      c.stats.qr_iterations++;
-      if (it < 16) c.stats.branch[it] = 1;
-      c.stats.flops += 4.0 * m * static_cast<double>(n) * n + static_cast<double>(n) * n * n;
-    }
-    ck(combine_update(m, n, X, ldx, Z.p, Z.ld, 0, 1, bkk, akk, nullptr, part, scal, c.stream()));
-    c.stats.launches += 2;
-    err = std::sqrt(d2h(c, scal));
-    if (it < 16) {
-      c.stats.con[it] = ckk;
-      c.stats.err[it] = err;
-      c.stats.ms_step[it] = tstep.stop();
-    }
-    ++it;
-    err2 = std::fabs(1.0 - lowk);
+    if (have != it && !read_back()) return false;
+    if (it > 0) err = std::sqrt(herr[std::min(it, kSlots) - 1]);
+    t_end = t_step.back();
+    for (int k = 0; k < std::min(it, 16); ++k) c.stats.ms_step[k] = marks.ms(t_step[k], t_step[k + 1]);
+    return true;
+  };
+  if (!iterate(false)) {
+    c.stats = stats0;
+    iterate(true);
   }
-  c.stats.ms_iter = ti.stop();
+  c.stats.ms_iter = marks.ms(t_loop, t_end);
   c.stats.iterations = it;
   c.stats.last_err = err;
   ck(scale_copy(m, n, 1.0, X, ldx, 0, dQ, ldq, 0, 1, 0.0, c.stream()));
   c.stats.launches++;
   if (dH) {
-    EventTimer th(c.stream());
+    const int t_h = marks.mark(c.stream());
     OzScope mixed_h(c, c.zolo_mixed >= 1);
     form_h(c, m, n, X, ldx, Ain, ldx, dH, ldh);
-    c.stats.ms_h = th.stop();
+    const int t_done = marks.mark(c.stream());
+    ck(cudaEventSynchronize(marks.ev[t_done]));
+    c.stats.ms_h = marks.ms(t_h, t_done);
   }
-  c.stats.ms_total = total.stop();
+  const int t_done = marks.mark(c.stream());
+  ck(cudaEventSynchronize(marks.ev[t_done]));
+  c.stats.ms_total = marks.ms(t_start, t_done);
   return mixed_status(c);
 }
 
@@ -555,15 +607,21 @@ int zolo_pd(Context& c, char sym, int rk, int m, int n, double alpha, double bet
   double con = 1.0 / beta, err = 1.0;
   int it = 0;
   const bool ns_finish = c.zolo_ns_finish != 0;
-  EventTimer ti(c.stream());
+  // with the Newton-Schulz finish ||X_{k+1} - X_k|| decides nothing: it stays on the device, a slot
+  // a step, and the step's time is read after the loop, so that no step ends in a wait
+  constexpr int kSlots = 16;
+  double* errs = scal + 32;
+  EventMarks marks;
+  std::vector<int> t_step{marks.mark(c.stream())};
   // term plan (ZOLO_OPT_TERM_PLAN): needs the measured Newton-Schulz finish to end the loop;
   // its coefficients come from the complementary modulus (exact at any CON)
   const bool plan_terms = ns_finish && c.zolo_term_plan && c.zolo_chol_inverse && !left;
   TermPlanner planner(rk, mx, n, tol, c.zolo_mixed >= 1);
   int planned = 0;
   // with the Newton-Schulz finish the loop ends at the measured check, not on ||X_{k+1} - X_k||
+  int finish_mark = -1;
   while ((ns_finish || err > tol2) && it < maxit) {
-    EventTimer tstep(c.stream());
+    double* err_slot = errs + std::min(it, kSlots - 1);
     int rk_it = rk;  // terms of this iteration
     if (plan_terms) rk_it = planned > 0 ? planned : planner.choose(con, it == 0 && pf && c.zolo_shared_qr);
     if (plan_terms) compute_coeff_kp(con, tol, rk_it, coeff.data());
@@ -589,7 +647,7 @@ int zolo_pd(Context& c, char sym, int rk, int m, int n, double alpha, double bet
             (!plan_terms || planner.predicts_finish(con) || planner.ns_cost(e0) <= planner.cost_from(con))) {
           newton_schulz_finish(c, mx, n, X, ldx, G, Z, e0, it);
           c.stats.ns_finish = 1;
-          c.stats.ms_finish = tstep.stop();
+          finish_mark = marks.mark(c.stream());
           break;
         }
       }
@@ -661,29 +719,40 @@ int zolo_pd(Context& c, char sym, int rk, int m, int n, double alpha, double bet
     }
     if (z_summed) {
       // Z already holds sum_j w_j Z_j / FONE
-      ck(combine_update(mx, n, X, ldx, Z.p, Z.ld, 0, 1, 1.0 / fone, 1.0, nullptr, part, scal, c.stream()));
+      ck(combine_update(mx, n, X, ldx, Z.p, Z.ld, 0, 1, 1.0 / fone, 1.0, nullptr, part, err_slot,
+                        c.stream()));
     } else {
       for (int b = 0; b < rk_it; ++b) hv[16 + b] /= fone;
       h2d(c, dvec + 16, hv.data() + 16, rk_it);
-      ck(combine_update(mx, n, X, ldx, Z.p, Z.ld, Z.stride, rk_it, 1.0 / fone, 0.0, dvec + 16, part, scal,
+      ck(combine_update(mx, n, X, ldx, Z.p, Z.ld, Z.stride, rk_it, 1.0 / fone, 0.0, dvec + 16, part, err_slot,
                         c.stream()));
     }
     c.stats.launches += 2;
     // plan the next iteration while this one runs
     if (plan_terms) planned = planner.choose(con_next, false);
-    err = std::sqrt(d2h(c, scal));
+    t_step.push_back(marks.mark(c.stream()));
+    if (!ns_finish) err = std::sqrt(d2h(c, err_slot));
     if (it < 16) {
       c.stats.con[it] = con;
-      c.stats.err[it] = err;
-      c.stats.ms_step[it] = tstep.stop();
       c.stats.terms[it] = rk_it;
     }
     con = con_next;
     ++it;
   }
-  c.stats.ms_iter = ti.stop();
-  c.stats.iterations = it;
-  c.stats.last_err = err;
+  const int t_iter = marks.mark(c.stream());
+  double herr[kSlots];
+  ck(cudaMemcpyAsync(herr, errs, sizeof(herr), cudaMemcpyDeviceToHost, c.stream()));
+  // once the stream has been waited for
+  auto finish_stats = [&]() {
+    c.stats.iterations = it;
+    for (int k = 0; k < std::min(it, 16); ++k) {
+      c.stats.err[k] = std::sqrt(herr[k]);
+      c.stats.ms_step[k] = marks.ms(t_step[k], t_step[k + 1]);
+    }
+    if (finish_mark >= 0) c.stats.ms_finish = marks.ms(t_step.back(), finish_mark);
+    c.stats.ms_iter = marks.ms(t_step[0], t_iter);
+    c.stats.last_err = it > 0 ? std::sqrt(herr[std::min(it, kSlots) - 1]) : err;
+  };
   OzScope mixed_h(c, c.zolo_mixed >= 1);  // forming Q and H
   if (factored) {
     EventTimer th(c.stream());  // ms_h covers Q = Q_x Y and H here
@@ -708,6 +777,7 @@ int zolo_pd(Context& c, char sym, int rk, int m, int n, double alpha, double bet
       c.stats.flops_exec_delta += dn * dn * dn - 2.0 * dm * dn * dn;
     }
     c.stats.ms_h = th.stop();
+    finish_stats();
     c.stats.ms_total = total.stop();
     return mixed_status(c);
   }
@@ -722,6 +792,7 @@ int zolo_pd(Context& c, char sym, int rk, int m, int n, double alpha, double bet
     c.stats.ms_h = th.stop();
   }
   c.stats.ms_total = total.stop();
+  finish_stats();
   return mixed_status(c);
 }
 
