@@ -52,3 +52,23 @@ def test_qdwh_cholesky_steps(h, n, sym):
     q, hh = zb.device_to_colmajor(dq), zb.device_to_colmajor(dh)
     assert zo.orthogonality(q) <= 10 * n * EPS + 4 * EPS
     assert zo.backward_error(a, q, hh) <= 10 * n * EPS + 4 * EPS
+
+
+# two leaves in one launch: one row to a full second leaf, and the levels above it; m > n, so no left solve
+@pytest.mark.parametrize("n", [66, 79, 80, 81, 96, 113, 127, 128, 129, 191, 193, 256, 385])
+def test_qdwh_paired_leaves(h, n):
+    import torch
+    m = n + 13
+    rng = np.random.default_rng(n)
+    u, _ = np.linalg.qr(rng.standard_normal((m, n)))
+    v, _ = np.linalg.qr(rng.standard_normal((n, n)))
+    a = (u * np.geomspace(1.0, 0.02, n)[None, :]) @ v.T
+    da = zb.colmajor_to_device(a)
+    dq, dh = torch.zeros_like(da), torch.zeros((n, n), dtype=torch.float64, device="cuda")
+    zb.qdwh_dev(h, "N", m, n, 0.0, da.data_ptr(), m, dq.data_ptr(), m, dh.data_ptr(), n, 0, 12, 0)
+    assert h.stats()["chol_iterations"] >= 2
+    q, hh = zb.device_to_colmajor(dq), zb.device_to_colmajor(dh)
+    assert zo.orthogonality(q) <= 10 * n * EPS
+    assert zo.backward_error(a, q, hh) <= 10 * n * EPS
+    # the polar factor is determined to kappa eps
+    assert np.linalg.norm(q - u @ v.T) <= 10 * n * EPS * 50

@@ -116,6 +116,10 @@ cudaError_t reduce_sum(const double* partial, int count, double* out, cudaStream
 // Dinv + b*strideD (nb x nb, ld ldd, zeros above the diagonal).
 cudaError_t potrf_leaf(int nb, double* A, int64_t lda, int64_t strideA, int batch, int* info,
                        int info_offset, double* Dinv, int64_t ldd, int64_t strideD, cudaStream_t st);
+// Y(b) = L^{-1} of the Cholesky factor of the nb x nb block at A(b), 64 < nb <= 128 (its 64 x 64 diagonal
+// blocks with the zeros above their diagonals); INFO as potrf_leaf.  A is not changed.
+cudaError_t potrf_inv_pair(int nb, const double* A, int64_t lda, int64_t strideA, int batch, int* info, int info_offset,
+                           double* Y, int64_t ldy, int64_t strideY, cudaStream_t st);
 // Inverses of all 64 x 64 diagonal blocks of lower-triangular n x n matrices:
 // block kb of batch entry b -> Dinv + b*strideD + kb*blk, ld ldd.
 cudaError_t trtri_blocks(int n, const double* L, int64_t ldl, int64_t strideL, double* Dinv, int64_t ldd, int64_t blk,

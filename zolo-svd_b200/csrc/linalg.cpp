@@ -226,6 +226,7 @@ static Mat block21(double* p, int n1, int n2) {
   const int64_t ld = (n2 + 1) / 2 * 2;
   return Mat{p, ld, ld * n1};
 }
+constexpr int kPairBatch = 16;
 static size_t block21_elems(int n) { return static_cast<size_t>(n / 2 + 1) * (n / 2 + 1); }
 
 // Cholesky and the inverse of its factor together: with Y11 = L11^{-1} from the first half,
@@ -241,7 +242,18 @@ static void potrf_inv_rec(Context& c, int n, Mat A, Mat Y, int batch, int* dinfo
     c.stats.launches++;
     return;
   }
-  const int n1 = split_point(n), n2 = n - n1;
+  // one CTA a member for two leaves, with most of an SM's shared memory: not where a batch keeps the
+  // SMs busy
+  const bool pair = batch <= kPairBatch;
+  if (pair && n <= 2 * NB) {
+    Profiler::Rec rec;
+    if (c.prof.on) c.prof.begin(2, 2.0 * n * n * n / 3.0 * batch, c.stream(), &rec);
+    ck(potrf_inv_pair(n, A.p, A.ld, A.stride, batch, dinfo, off, Y.p, Y.ld, Y.stride, c.stream()));
+    if (c.prof.on) c.prof.end(rec, c.stream());
+    c.stats.launches++;
+    return;
+  }
+  const int n1 = pair ? (n / 2 + 2 * NB - 1) / (2 * NB) * (2 * NB) : split_point(n), n2 = n - n1;
   potrf_inv_rec(c, n1, A, Y, batch, dinfo, off, tmp);
   const Mat Tmp = block21(tmp, n1, n2);
   // Y11^T is upper triangular (k up to the column), Y11 lower (k from the column)

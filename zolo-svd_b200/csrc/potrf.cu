@@ -179,22 +179,16 @@ ZDEV void load_leaf(int nb, const double* A, int64_t lda, double* a, double* x) 
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(PT) potrf_leaf_kernel(int nb, double* A, int64_t lda, int64_t strideA, int* info,
-                                                        int info_offset, double* Dinv, int64_t ldd, int64_t strideD) {
-  extern __shared__ double sm[];
-  double* a = sm;
-  double* x = sm + LEAF * LDS;
-  double* Ab = A + blockIdx.x * strideA;
+// Factor of the leaf in a (all warps; identity beyond nb) and the inverses of its 16 x 16 diagonal
+// blocks in x, ones on x's diagonal past the eliminated blocks.
+ZDEV void factor_leaf(int nb, double* a, double* x, double* piv, int* info, int info_offset) {
   const int warp = threadIdx.x >> 5;
-  __shared__ __align__(16) double piv[4 * LB];
-  dependency_wait();
-  load_leaf(nb, Ab, lda, a, x);
   const int n16 = (nb + LB - 1) / LB * LB;  // identity blocks past nb need no elimination
   for (int k0 = 0; k0 < n16; k0 += LB) {
     if (warp == 0) {
       const int bad = factor_block(a, x, k0, piv);
       if (bad && threadIdx.x == 0 && info && k0 + bad <= nb)  // LAPACK INFO = first non-positive pivot
-        atomicCAS(info + blockIdx.x, 0, info_offset + k0 + bad);
+        atomicCAS(info, 0, info_offset + k0 + bad);
     }
     __syncthreads();
     const int rows = (n16 - k0 - LB) / 16;  // 16-row tiles below
@@ -224,19 +218,110 @@ __global__ void __launch_bounds__(PT) potrf_leaf_kernel(int nb, double* A, int64
     }
     __syncthreads();
   }
+  for (int i = n16 + threadIdx.x; i < LEAF; i += PT) x[i + i * LDS] = 1.0;
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(PT) potrf_leaf_kernel(int nb, double* A, int64_t lda, int64_t strideA, int* info,
+                                                        int info_offset, double* Dinv, int64_t ldd, int64_t strideD) {
+  extern __shared__ double sm[];
+  double* a = sm;
+  double* x = sm + LEAF * LDS;
+  double* Ab = A + blockIdx.x * strideA;
+  __shared__ __align__(16) double piv[4 * LB];
+  dependency_wait();
+  load_leaf(nb, Ab, lda, a, x);
+  factor_leaf(nb, a, x, piv, info ? info + blockIdx.x : nullptr, info_offset);
   for (int e = threadIdx.x; e < LEAF * LEAF; e += PT) {
     const int i = e & (LEAF - 1), j = e >> 6;
     if (i < nb && j <= i) Ab[i + j * lda] = a[i + j * LDS];
-    if (i >= n16 && i == j) x[i + j * LDS] = 1.0;
   }
   release_dependents();
   if (!Dinv) return;
-  __syncthreads();
+  __syncthreads();  // the factor is read: the merge uses its upper triangle
   merge_inverse(a, x);
   double* Db = Dinv + blockIdx.x * strideD;
   for (int e = threadIdx.x; e < LEAF * LEAF; e += PT) {
     const int i = e & (LEAF - 1), j = e >> 6;
     if (i < nb && j < nb) Db[i + j * ldd] = x[i + j * LDS];
+  }
+}
+
+// Y = L^{-1} of the Cholesky factor of a block of 64 < nb <= 128 rows, one CTA: two leaves with
+// their inverses, L21 = A21 X11^T, A22 - L21 L21^T, X21 = -X22 (L21 X11), all in shared memory.  As two
+// leaf launches and four products of 64 x 64 tiles on a few SMs it was 57 us; the chain of 128 pivots
+// and the products are 41 us here (QDWH n = 1024 9.23 -> 9.05 ms).  The factor is not written back.
+__global__ void __launch_bounds__(PT) potrf_inv_pair_kernel(int nb, const double* A, int64_t lda, int64_t strideA,
+                                                            int* info, int info_offset, double* Y, int64_t ldy,
+                                                            int64_t strideY) {
+  extern __shared__ double sm[];
+  constexpr int BLK = LEAF * LDS;
+  double *a11 = sm, *x11 = sm + BLK, *a21 = sm + 2 * BLK, *a22 = sm + 3 * BLK, *x22 = sm + 4 * BLK, *l21 = sm + 5 * BLK;
+  __shared__ __align__(16) double piv[4 * LB];
+  const double* Ab = A + blockIdx.x * strideA;
+  int* inf = info ? info + blockIdx.x : nullptr;
+  const int warp = threadIdx.x >> 5, nb2 = nb - LEAF;
+  dependency_wait();
+  {
+    constexpr int NE = LEAF * LEAF / PT;
+    double v[NE];
+#pragma unroll
+    for (int q = 0; q < NE; ++q) {
+      const int e = threadIdx.x + q * PT, i = e & (LEAF - 1), j = e >> 6;
+      v[q] = i < nb2 ? Ab[LEAF + i + j * lda] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < NE; ++q) {
+      const int e = threadIdx.x + q * PT;
+      a21[(e & (LEAF - 1)) + (e >> 6) * LDS] = v[q];
+    }
+  }
+  load_leaf(nb2, Ab + LEAF + LEAF * lda, lda, a22, x22);
+  load_leaf(LEAF, Ab, lda, a11, x11);
+  factor_leaf(LEAF, a11, x11, piv, inf, info_offset);
+  merge_inverse(a11, x11);
+  for (int u = warp; u < 32; u += PT / 32) {  // L21: column tile tj of X11^T needs k < 8 tj + 8
+    const int ti = u & 3, tj = u >> 2;
+    double c[4] = {0.0, 0.0, 0.0, 0.0};
+    tile_mma<true>(c, a21 + 16 * ti, x11 + 8 * tj, 8 * tj + 8);
+    tile_store(l21 + 16 * ti + 8 * tj * LDS, c, 1.0);
+  }
+  __syncthreads();
+  for (int u = warp; u < 52; u += PT / 32) {
+    double c[4] = {0.0, 0.0, 0.0, 0.0};
+    if (u < 20) {  // A22 - L21 L21^T on the tiles meeting the lower triangle
+      int ti = 0, r = u;
+      while (r >= 2 * ti + 2) {
+        r -= 2 * ti + 2;
+        ++ti;
+      }
+      tile_mma<true>(c, l21 + 16 * ti, l21 + 8 * r, LEAF);
+      tile_sub(a22 + 16 * ti + 8 * r * LDS, c);
+    } else {  // L21 X11 over A21: X11's column tile starts at row 8 tj
+      const int ti = (u - 20) & 3, k0 = ((u - 20) >> 2) * 8;
+      tile_mma<false>(c, l21 + 16 * ti + k0 * LDS, x11 + k0 + k0 * LDS, LEAF - k0);
+      tile_store(a21 + 16 * ti + k0 * LDS, c, 1.0);
+    }
+  }
+  __syncthreads();
+  factor_leaf(nb2, a22, x22, piv, inf, info_offset + LEAF);
+  merge_inverse(a22, x22);
+  for (int u = warp; u < 32; u += PT / 32) {
+    const int ti = u & 3, tj = u >> 2;
+    double c[4] = {0.0, 0.0, 0.0, 0.0};
+    tile_mma<false>(c, x22 + 16 * ti, a21 + 8 * tj * LDS, 16 * ti + 16);
+    tile_store(l21 + 16 * ti + 8 * tj * LDS, c, -1.0);
+  }
+  release_dependents();
+  __syncthreads();
+  double* Yb = Y + blockIdx.x * strideY;
+  for (int e = threadIdx.x; e < LEAF * LEAF; e += PT) {
+    const int i = e & (LEAF - 1), j = e >> 6, o = i + j * LDS;
+    Yb[i + j * ldy] = x11[o];
+    if (i < nb2) {
+      Yb[LEAF + i + j * ldy] = l21[o];
+      if (j < nb2) Yb[LEAF + i + (LEAF + j) * ldy] = x22[o];
+    }
   }
 }
 
@@ -265,6 +350,7 @@ __global__ void __launch_bounds__(PT) trtri_blocks_kernel(int n, const double* L
 }
 
 constexpr int SMEM_BYTES = 2 * LEAF * LDS * 8;
+constexpr int SMEM_PAIR = 6 * LEAF * LDS * 8;
 
 }  // namespace
 
@@ -279,6 +365,19 @@ cudaError_t potrf_leaf(int nb, double* A, int64_t lda, int64_t strideA, int batc
   if (attr != cudaSuccess) return attr;
   return launch_dependent(potrf_leaf_kernel, dim3(batch), dim3(PT), SMEM_BYTES, st, dim3(1), nb, A, lda, strideA, info,
                           info_offset, Dinv, ldd, strideD);
+}
+
+cudaError_t potrf_inv_pair(int nb, const double* A, int64_t lda, int64_t strideA, int batch, int* info, int info_offset,
+                           double* Y, int64_t ldy, int64_t strideY, cudaStream_t st) {
+  if (batch <= 0) return cudaSuccess;
+  if (nb <= LEAF || nb > 2 * LEAF) return cudaErrorInvalidValue;
+  static std::atomic<int> attr_set[kMaxDevices];
+  const cudaError_t attr = once_per_device(attr_set, [] {
+    return cudaFuncSetAttribute(potrf_inv_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PAIR);
+  });
+  if (attr != cudaSuccess) return attr;
+  return launch_dependent(potrf_inv_pair_kernel, dim3(batch), dim3(PT), SMEM_PAIR, st, dim3(1), nb, A, lda, strideA, info,
+                          info_offset, Y, ldy, strideY);
 }
 
 cudaError_t trtri_blocks(int n, const double* L, int64_t ldl, int64_t strideL, double* Dinv, int64_t ldd, int64_t blk,
