@@ -60,3 +60,36 @@ def test_structured(h, m, n, pad):
     assert bool((torch.linalg.norm(q @ r - da, dim=0) <= 10 * n * EPS * torch.linalg.norm(da, dim=0)).all())
     assert float(torch.linalg.norm(q.T @ q - torch.eye(n, dtype=torch.float64, device="cuda"))) <= 10 * n * EPS
     assert bool((torch.tril(q[m:], -1) == 0.0).all())
+
+
+# blocks of 128 columns, the last one with one to four panels and a ragged last panel (its T by pairs of panels)
+@pytest.mark.parametrize("w", [1, 31, 32, 33, 64, 65, 96, 97, 127, 128])
+def test_block_t(h, w):
+    import torch
+    m, n = 8192, 640 + w
+    g = torch.Generator(device="cuda")
+    g.manual_seed(w)
+    da = torch.randn((m, n), dtype=torch.float64, device="cuda", generator=g)
+    q, r = _run(h, da.cpu().numpy(), 0, -1)
+    assert bool((torch.linalg.norm(q @ r - da, dim=0) <= 10 * n * EPS * torch.linalg.norm(da, dim=0)).all())
+    assert float(torch.linalg.norm(q.T @ q - torch.eye(n, dtype=torch.float64, device="cuda"))) <= 10 * n * EPS
+
+
+# the mixed form applies Q in blocks of 512 columns: one block, one and a ragged rest, two
+@pytest.mark.parametrize("n", [300, 511, 513, 640, 700, 1024, 1100])
+def test_wide_blocks(n):
+    import torch
+    m = n + 37
+    hd = zb.Handle(0)
+    for o in (zb.OPT_NS_FINISH, zb.OPT_CHOL_INVERSE, zb.OPT_BETA_FROB, zb.OPT_TERM_PLAN, zb.OPT_MIXED):
+        hd.set_option(o, 1)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    a = torch.randn((m, n), dtype=torch.float64, device="cuda", generator=g)
+    da = a.T.contiguous()
+    dq, dh = torch.zeros_like(da), torch.zeros((n, n), dtype=torch.float64, device="cuda")
+    zb.polar_dev(hd, 8, m, n, da.data_ptr(), m, dq.data_ptr(), m, dh.data_ptr(), n)
+    q, hh = dq.T, dh.T
+    assert float(torch.linalg.norm(q.T @ q - torch.eye(n, dtype=torch.float64, device="cuda"))) <= 10 * n * EPS
+    assert float(torch.linalg.norm(q @ hh - a) / torch.linalg.norm(a)) <= 10 * n * EPS
+    hd.close()

@@ -142,10 +142,10 @@ int qr_panel_config(int m, int w);
 cudaError_t extract_v(int m, int w, const double* A, int64_t lda, int64_t strideA, double* V,
                       int64_t ldv, int64_t strideV, int batch, cudaStream_t st, int split = 0,
                       int64_t gap = 0);
-// TB(b) (jb x jb, ld ldtb) <- block diagonal of the ceil(jb/32) consecutive 32 x 32 panel T
-// factors at T + b*strideT (ld 32, 1024 apart), zero elsewhere.
-cudaError_t block_t_init(int jb, const double* T, int64_t strideT, double* TB, int64_t ldtb, int64_t strideTB,
-                         int batch, cudaStream_t st);
+// TB(b) (jb x jb, ld ldtb) <- the block reflectors' T of every 128 columns, from the ceil(jb/32) panel T
+// factors at T + b*strideT (32 x 32, ld 32, 1024 apart) and the lower triangle G of V^T V; zero elsewhere.
+cudaError_t block_t_merge(int jb, const double* T, int64_t strideT, const double* G, int64_t ldg, int64_t strideG,
+                          double* TB, int64_t ldtb, int64_t strideTB, int batch, cudaStream_t st);
 // P'(b) = T(b)^T * P(b) (trans=1) or T(b) * P(b) (trans=0); T w x w upper (ld 32), P w x n.
 cudaError_t apply_t(int w, int n, const double* T, int64_t strideT, double* P, int64_t ldp,
                     int64_t strideP, int trans, int batch, cudaStream_t st);

@@ -365,23 +365,25 @@ static void panel_b_minus_vp(Context& c, const PanelRows& R, int jb, int ncols, 
 }
 
 // T_B (jb x jb upper) of the block reflector I - V_B T_B V_B^T = H_1 H_2 ... of the block's
-// 32-column panels (the compact WY recursion of LAPACK DLARFT, by panels): the diagonal
-// blocks are the panels' T, and T_B(0:c0, q) = -T_B(0:c0, 0:c0) (V_B(:, 0:c0)^T V_q) T_q.
+// 32-column panels (the compact WY form of LAPACK DLARFT, by pairs of panels): with the panels' T on the
+// diagonal, T12 = -T1 (V1^T V2) T2, up to 128 columns in one launch, wider pairs by products.
 // VB: the block's explicit V, mp packed rows.  T: the first panel's T (32 x 32 per panel).
 static void block_t(Context& c, int jb, Mat VB, int mp, const double* T, int64_t strideT, Mat TB, int batch) {
-  const int ldg = std::max(jb, 2);
+  const int ldg = (std::max(jb, 2) + 1) / 2 * 2;
   Mat G{c.buf("qr_bg", static_cast<size_t>(ldg) * ldg * batch), ldg, static_cast<int64_t>(ldg) * ldg};
-  Mat Tmp{c.buf("qr_btmp", static_cast<size_t>(ldg) * PW * batch), ldg, static_cast<int64_t>(ldg) * PW};
   // lower triangle of V_B^T V_B: its transpose gives the blocks above the diagonal
   gemm(c, 1, 0, jb, jb, mp, 1.0, VB, VB, 0.0, G, batch, nullptr, 1, 0);
-  ck(block_t_init(jb, T, strideT, TB.p, TB.ld, TB.stride, batch, c.stream()));
+  ck(block_t_merge(jb, T, strideT, G.p, G.ld, G.stride, TB.p, TB.ld, TB.stride, batch, c.stream()));
   c.stats.launches++;
-  for (int c0 = PW; c0 < jb; c0 += PW) {
-    const int w = std::min(PW, jb - c0);
-    // Tmp = T_B(0:c0, 0:c0) G(c0:c0+w, 0:c0)^T  (T_B upper: k from the row)
-    gemm(c, 0, 1, c0, w, c0, 1.0, TB, G.at(c0, 0), 0.0, Tmp, batch, nullptr, 0, 2);
-    gemm(c, 0, 0, c0, w, w, -1.0, Tmp, TB.at(c0, c0), 0.0, TB.at(0, c0), batch);
-  }
+  if (jb <= QB) return;
+  Mat Tmp{c.buf("qr_btmp", static_cast<size_t>(ldg) * ldg * batch), ldg, static_cast<int64_t>(ldg) * ldg};
+  for (int s = QB; s < jb; s *= 2)
+    for (int o = 0; o + s < jb; o += 2 * s) {
+      const int w = std::min(s, jb - o - s);
+      // T1 upper (k from the row), T2 upper (k up to the column)
+      gemm(c, 0, 1, s, w, s, 1.0, TB.at(o, o), G.at(o + s, o), 0.0, Tmp, batch, nullptr, 0, 2);
+      gemm(c, 0, 0, s, w, w, -1.0, Tmp, TB.at(o + s, o + s), 0.0, TB.at(o, o + s), batch, nullptr, 0, 0, nullptr, 2);
+    }
 }
 
 // C <- (I - V op(T) V^T) C over the panel's rows, V the panel at Vp in the factored matrix and C the

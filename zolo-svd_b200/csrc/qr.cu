@@ -698,21 +698,109 @@ __global__ void extract_v_kernel(int m, int w, const double* __restrict__ A, int
   });
 }
 
-// TB (jb x jb) <- the block diagonal of consecutive panels' T factors (QW x QW each, ld QW,
-// QW*QW apart), zero elsewhere: the diagonal of the block reflector's T.
-__global__ void block_t_init_kernel(int jb, const double* __restrict__ T, int64_t strideT, double* TB,
-                                    int64_t ldtb, int64_t strideTB) {
-  dependency_wait();
-  release_dependents();
-  const double* Tb = T + blockIdx.y * strideT;
-  double* Bb = TB + blockIdx.y * strideTB;
-  const int total = jb * jb;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-    const int i = e % jb, j = e / jb;
-    const int q = i / QW;
-    const double v = (q == j / QW && i <= j) ? Tb[q * QW * QW + (i % QW) + (j % QW) * QW] : 0.0;
-    Bb[i + static_cast<int64_t>(j) * ldtb] = v;
+// T of up to four panels' block reflector from their T factors and the lower triangle of V^T V:
+// T12 = -T1 (V1^T V2) T2 for pairs of 32 columns, then of 64, in one CTA's shared memory (both
+// products on the FP64 tensor path).  One array holds T in its upper triangle and V^T V strictly below the
+// panels' diagonal blocks.  blockIdx.x: the 128-column block of TB; the CTA writes its columns, zero
+// outside its own rows.  Bound by latency: 7 us (25 with the loads in eight dependent rounds), where the
+// set-up and six small products of the panel-by-panel recursion were a chain of 30 us.
+constexpr int BTW = 128, BTT = 512;
+constexpr int BTL = BTW + 4, BTP = 64 + 4;  // = 4 mod 16: conflict-free fragment loads
+template <bool TB, int LDB>
+ZDEV void bt_mma(double (&c)[4], const double* a, int lda, const double* b, int K) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll 4
+  for (int k = 0; k < K; k += 8) {
+    double af[4], bf[2];
+    af[0] = a[g + (k + t) * lda];
+    af[1] = a[g + 8 + (k + t) * lda];
+    af[2] = a[g + (k + t + 4) * lda];
+    af[3] = a[g + 8 + (k + t + 4) * lda];
+    bf[0] = TB ? b[g + (k + t) * LDB] : b[k + t + g * LDB];
+    bf[1] = TB ? b[g + (k + t + 4) * LDB] : b[k + t + 4 + g * LDB];
+    dmma_16x8x8(c, af, bf);
   }
+}
+ZDEV void bt_store(double* s, int ld, const double (&c)[4], double alpha) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  s[g + (2 * t) * ld] = alpha * c[0];
+  s[g + (2 * t + 1) * ld] = alpha * c[1];
+  s[g + 8 + (2 * t) * ld] = alpha * c[2];
+  s[g + 8 + (2 * t + 1) * ld] = alpha * c[3];
+}
+
+__global__ void __launch_bounds__(BTT) block_t_kernel(int jb, const double* T, int64_t strideT, const double* G,
+                                                      int64_t ldg, int64_t strideG, double* TB, int64_t ldtb,
+                                                      int64_t strideTB) {
+  extern __shared__ __align__(16) double bt_sm[];
+  double* S = bt_sm;
+  double* P = bt_sm + BTW * BTL;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int c0 = blockIdx.x * BTW, w = min(BTW, jb - c0);
+  const double* Tb = T + blockIdx.y * strideT + static_cast<int64_t>(c0 / QW) * QW * QW;
+  const double* Gb = G + blockIdx.y * strideG + c0 + c0 * ldg;
+  double* Bb = TB + blockIdx.y * strideTB + c0 * ldtb;
+  dependency_wait();
+  {
+    // the panels' T and the six blocks of V^T V below them, pairs of rows, all loads in flight together
+    constexpr int NT2 = 4 * QW * QW / 2 / BTT, NG2 = 6 * QW * QW / 2 / BTT;
+    double2 vt[NT2], vg[NG2];
+    int og[NG2];
+#pragma unroll
+    for (int x = 0; x < NT2; ++x) {
+      const int e = (tid + x * BTT) * 2, q = e / (QW * QW);
+      vt[x] = q * QW < w ? make_double2(Tb[e], Tb[e + 1]) : make_double2(0.0, 0.0);
+    }
+#pragma unroll
+    for (int x = 0; x < NG2; ++x) {
+      const int e = (tid + x * BTT) * 2, blk = e / (QW * QW), r = e % (QW * QW);
+      const int bi = blk == 0 ? 1 : (blk <= 2 ? 2 : 3), bj = blk - bi * (bi - 1) / 2;
+      const int i = bi * QW + r % QW, j = bj * QW + r / QW;
+      const double* src = Gb + i + j * ldg;
+      og[x] = i + j * BTL;
+      vg[x] = make_double2(i < w ? src[0] : 0.0, i + 1 < w ? src[1] : 0.0);
+    }
+#pragma unroll
+    for (int x = 0; x < NT2; ++x) {
+      const int e = (tid + x * BTT) * 2, q = e / (QW * QW), r = e % (QW * QW);
+      *reinterpret_cast<double2*>(S + q * QW + r % QW + (q * QW + r / QW) * BTL) = vt[x];
+    }
+#pragma unroll
+    for (int x = 0; x < NG2; ++x) *reinterpret_cast<double2*>(S + og[x]) = vg[x];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int h = QW; h < BTW; h *= 2) {
+    const int rt = h / 16, ct = h / 8, per = rt * ct, pairs = BTW / (2 * h);  // 16 x 8 tiles of a pair's T12
+    if (w <= h) break;
+    for (int u = warp; u < pairs * per; u += BTT / 32) {  // P = T1 (V2^T V1)^T, T1 upper: k from the row
+      const int p = u / per, o = p * 2 * h, ti = (u % per) / ct * 16, tj = (u % per) % ct * 8;
+      double c[4] = {0.0, 0.0, 0.0, 0.0};
+      bt_mma<true, BTL>(c, S + o + ti + (o + ti) * BTL, BTL, S + o + h + tj + (o + ti) * BTL, h - ti);
+      bt_store(P + p * h + ti + tj * BTP, BTP, c, 1.0);
+    }
+    __syncthreads();
+    for (int u = warp; u < pairs * per; u += BTT / 32) {  // T12 = -P T2, T2 upper: k up to the column
+      const int p = u / per, o = p * 2 * h, ti = (u % per) / ct * 16;
+      const int cj = u >= BTT / 32 ? ct - 1 - (u % per) % ct : (u % per) % ct, tj = cj * 8;
+      double c[4] = {0.0, 0.0, 0.0, 0.0};
+      bt_mma<false, BTL>(c, P + p * h + ti, BTP, S + o + h + (o + h + tj) * BTL, tj + 8);
+      bt_store(S + o + ti + (o + h + tj) * BTL, BTL, c, -1.0);
+    }
+    // V2^T V1 of these pairs is used up: T is upper triangular to the next level
+    for (int e = tid; e < pairs * h * h; e += BTT) {
+      const int p = e / (h * h), i = e % h, j = e / h % h;
+      S[p * 2 * h + h + i + (p * 2 * h + j) * BTL] = 0.0;
+    }
+    __syncthreads();
+  }
+  release_dependents();
+  // zeros below the diagonal, and beside the block when jb has more than one
+  for (int j = warp; j < w; j += BTT / 32)
+    for (int i = tid & 31; i < jb; i += 32) {
+      const int l = i - c0;
+      Bb[i + j * ldtb] = l >= 0 && l <= j ? S[l + j * BTL] : 0.0;
+    }
 }
 
 // P(:,col) <- T^T P(:,col)  or  T P(:,col), T upper triangular w x w (ld QW)
@@ -907,11 +995,17 @@ cudaError_t extract_v(int m, int w, const double* A, int64_t lda, int64_t stride
   return launch_dependent(extract_v_kernel, dim3(blocks, batch), dim3(256), 0, st, dim3(1), m, w, A, lda, strideA, V, ldv, strideV, split, gap);
 }
 
-cudaError_t block_t_init(int jb, const double* T, int64_t strideT, double* TB, int64_t ldtb, int64_t strideTB,
-                         int batch, cudaStream_t st) {
+cudaError_t block_t_merge(int jb, const double* T, int64_t strideT, const double* G, int64_t ldg, int64_t strideG,
+                          double* TB, int64_t ldtb, int64_t strideTB, int batch, cudaStream_t st) {
   if (jb <= 0 || batch <= 0) return cudaSuccess;
-  const int blocks = (jb * jb + 255) / 256;
-  return launch_dependent(block_t_init_kernel, dim3(blocks, batch), dim3(256), 0, st, dim3(1), jb, T, strideT, TB, ldtb, strideTB);
+  constexpr int smem = (BTW * BTL + 64 * BTP) * 8;
+  static std::atomic<int> attr_set[kMaxDevices];
+  const cudaError_t attr = once_per_device(attr_set, [] {
+    return cudaFuncSetAttribute(block_t_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  });
+  if (attr != cudaSuccess) return attr;
+  return launch_dependent(block_t_kernel, dim3((jb + BTW - 1) / BTW, batch), dim3(BTT), smem, st, dim3(1), jb, T,
+                          strideT, G, ldg, strideG, TB, ldtb, strideTB);
 }
 
 cudaError_t apply_t(int w, int n, const double* T, int64_t strideT, double* P, int64_t ldp, int64_t strideP,
