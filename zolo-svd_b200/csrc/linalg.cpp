@@ -401,10 +401,12 @@ static void apply_panel(Context& c, const PanelRows& R, int jb, int ncols, Mat V
 // Factorizations that apply every panel to all remaining columns at once (apply_panel) instead of
 // in 128-column blocks: while the trailing update fits beside the next panel the blocks' T factors
 // and products only lengthen the chain.  Measured, panelwise against blocks: QR of 1024 x 1024
-// 1.6 / 2.0 ms, 2048 x 2048 4.0 / 4.7, 4096 x 2048 8.2 / 6.3; forming Q, where nothing hides the
-// update, 1024 x 1024 0.48 / 0.63 ms, 2048 x 1024 0.93 / 0.80.
+// 1.52 / 1.67 ms, 2048 x 2048 3.71 / 4.04, 4096 x 2048 7.6 / 5.7; forming Q, where nothing hides the
+// update, 512 x 512 0.147 / 0.157, 1024 x 1024 0.42 / 0.38, 2048 x 1024 0.86 / 0.55.  A batch of
+// 64 matrices of n <= 160 takes 1.73 ms with its buckets up to 1.5e6 panelwise, 1.77 with 5e5.
 static bool panelwise(int mtot, int n, int batch, bool qr) {
-  return reflect_applies(mtot) && static_cast<double>(mtot) * n * batch <= (qr ? 4.5e6 : 1.5e6);
+  const double one = static_cast<double>(mtot) * n, all = one * batch;
+  return reflect_applies(mtot) && (qr ? all <= 4.5e6 : one <= 5e5 && all <= 1.5e6);
 }
 
 static void factor_panel(Context& c, int mtot, int n, int m_top, bool top_tri, int j, Mat W, double* tau, double* T,

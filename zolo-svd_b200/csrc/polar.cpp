@@ -499,6 +499,7 @@ int qdwh(Context& c, int m, int n, const double* dA, int64_t lda, double* dQ, in
           if (it < 16) c.stats.branch[it] = 2;
           c.stats.flops += 2.0 * m * static_cast<double>(n) * n + static_cast<double>(n) * n * n / 3.0 +
                            static_cast<double>(m) * n * n;
+          c.stats.flops_exec_delta += static_cast<double>(n) * n * n / 3.0;  // the factor's inverse
         }
       }
       if (use_qr) {
@@ -689,6 +690,7 @@ int zolo_pd(Context& c, char sym, int rk, int m, int n, double alpha, double bet
         if (it < 16) c.stats.branch[it] = 2;
         c.stats.flops += static_cast<double>(m) * n * n +
                          rk_it * (static_cast<double>(n) * n * n / 3.0 + 2.0 * m * static_cast<double>(n) * n);
+        c.stats.flops_exec_delta += rk_it * static_cast<double>(n) * n * n / 3.0;  // the factors' inverses
       }
     }
     const double fone = zolo_fone(coeff.data(), rk_it);
@@ -983,7 +985,7 @@ void qdwh_bucket(Context& c, const std::vector<int>& idx, int MB, int NB, const 
   };
   auto count_step = [&](bool qr, const std::vector<char>& active) {
     flops += B * (qr ? 4.0 * MB * static_cast<double>(NB) * NB + static_cast<double>(NB) * NB * NB
-                     : 2.0 * MB * static_cast<double>(NB) * NB + NB * static_cast<double>(NB) * NB / 3.0 +
+                     : 2.0 * MB * static_cast<double>(NB) * NB + 2.0 * NB * static_cast<double>(NB) * NB / 3.0 +
                            static_cast<double>(MB) * NB * NB);
     for (int b = 0; b < B; ++b) {
       if (!active[b]) continue;
