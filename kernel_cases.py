@@ -9,7 +9,7 @@ solve (e.g. ``ncu -k regex:dgemm_kernel ... python kernel_cases.py --case gemm_n
 
   gemm_nn      C = A B, M = N = K = n          (general DMMA GEMM, 128 x 128 tiles)
   gemm_rank32  C -= A B, M = N = n, K = 32     (streaming rank-32 update kernel)
-  gemm_k128    C -= A B, M = N = n, K = 128    (block-reflector update, 64 x 64 tiles, C preloaded)
+  gemm_k128    C -= A B, M = N = n, K = 128    (block-reflector update, 64 x 64 tiles, C staged)
   gemm_m32     P = V^T W, M = 32, N = K = n    (panel projection, 32 x 64 tiles)
   syrk         lower(C) = A^T A, n x n          (Gram of the Cholesky form)
   geqrf        Householder QR of an n x n matrix (panel kernel + trailing GEMMs)

@@ -98,7 +98,7 @@ class Context {
   int zolo_shared_qr = 1;
   // Zolo-PD stopping: 0 = reference rule, 1 = Newton-Schulz finish once ||X^T X - I|| is small.
   int zolo_ns_finish = 0;
-  // Zolo-PD Cholesky iterations: 0 = two triangular solves per term (zolochol.f90),
+  // Zolo-PD Cholesky iterations: 0 = two products with L^-T and L^-1 per term (zolochol.f90),
   // 1 = explicit inverses summed into S, then one Z = X S.
   int zolo_chol_inverse = 0;
   // zolo_polar's bounds: 0 = beta = 1/(sqrt(n) ||R^-1||_1) (test_zolodrv1.f90), 1 = 1/||R^-1||_F.
