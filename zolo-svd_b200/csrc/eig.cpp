@@ -212,13 +212,26 @@ struct Presolved {
   int info = 1;
 };
 
+// Leak of a split, ||V2^T H V1||_F in units of eps sqrt(m) ||H||_F, up to which the first subspace pass of
+// an m x m node of an n x n problem stands: 10, and less where leaks of that size at every node of
+// the L levels above the leaves, sqrt(2 L n) of them in ||A - U S V^T||_F, would pass 1e-13 ||A||_F (1.3 at
+// n = 8192, 2 at 4096, 6 at 701).  With 10 for every n a leak of 9.2 at the root of 16384 x 8192 stood and
+// left 2.6e-13; the second pass there leaves 1.9e-14 and takes 3.04 s to 3.12.  The mixed form reads the
+// leak through INT8-emulated products, whose own rounding is 1.2 at n = 8192: at least 2, or further
+// passes are spent on it.
+double leak_line(int n, bool mixed) {
+  const double eps = 2.220446049250313e-16;
+  const double levels = std::max(1.0, std::ceil(std::log2(static_cast<double>(n) / kJacobiLeaf)));
+  return std::clamp(1e-13 / (std::sqrt(2.0 * levels * n) * eps), mixed ? 2.0 : 0.0, 10.0);
+}
+
 // One node of the divide-and-conquer: a leaf (m <= kJacobiLeaf) or a split into the blocks of
 // V^T H V above and below a shift (QDWH polar factor of H - sigma I, subspace basis of its
 // projector).  Fills nd (k, V, Z, w) and the children L, R; returns false if no candidate
 // shift splits the spectrum.  dg: the node's diagonal (empty for a leaf); pre: the first
-// candidate's polar factor when already computed.
-bool split_node(Context& c, Node& nd, Node& L, Node& R, DevMem& mem, double hnorm, uint64_t seed, EigStats& S,
-                const std::vector<double>& dg, const Presolved& pre) {
+// candidate's polar factor when already computed; leak: leak_line.
+bool split_node(Context& c, Node& nd, Node& L, Node& R, DevMem& mem, double hnorm, double leak, uint64_t seed,
+                EigStats& S, const std::vector<double>& dg, const Presolved& pre) {
   const double eps = 2.220446049250313e-16;
   const int m = nd.n;
   const int64_t ldm = even(m);
@@ -283,7 +296,7 @@ bool split_node(Context& c, Node& nd, Node& L, Node& R, DevMem& mem, double hnor
       gemm(c, 0, 0, m, k, m, 1.0, Mat{P, ldm, 0}, Mat{Om, ldm, 0}, 0.0, Mat{X, ldm, 0}, 1);
     }
     basis_from(c, m, k, Mat{X, ldm, 0}, nd.V, ldm);
-    const double tol = 10.0 * eps * std::sqrt(static_cast<double>(m)) * std::max(hnorm, 1e-300);
+    const double tol = leak * eps * std::sqrt(static_cast<double>(m)) * std::max(hnorm, 1e-300);
     double off = split_residual(c, m, k, nd.H, nd.ld, nd.V, ldm, E, ldm, true);
     S.subspace_passes++;
     for (int pass = 1; pass < 3 && off > tol; ++pass) {
@@ -340,6 +353,7 @@ int syev_dc(Context& c, int n, const double* dH, int64_t ldh, double* dW, double
   double hnorm;
   ck(frob2(n, n, nodes[0].H, nodes[0].ld, c.dpartial(), c.dscal() + 9, c.stream()));
   hnorm = std::sqrt(d2h(c, c.dscal() + 9));
+  const double leak = leak_line(n, c.zolo_mixed >= 1);
 
   // ---- top-down splits, one level at a time: the nodes of a level run concurrently ----
   std::vector<std::pair<size_t, size_t>> levels;
@@ -446,7 +460,7 @@ int syev_dc(Context& c, int n, const double* dH, int64_t ldh, double* dW, double
     std::vector<double> cost(cnt);
     for (int i = 0; i < cnt; ++i) cost[i] = std::pow(static_cast<double>(nodes[lo + i].n), 3);
     run_concurrent(c, cnt, cost, [&](Context& wc, int i) {
-      ok[i] = split_node(wc, nodes[lo + i], kids[2 * i], kids[2 * i + 1], mem, hnorm,
+      ok[i] = split_node(wc, nodes[lo + i], kids[2 * i], kids[2 * i + 1], mem, hnorm, leak,
                          0x5EEDull + (lo + i) * 7919ull, st[i], dg[i], pre[i]) ? 1 : 0;
     });
     S.wall_split += wall_ms_since(w0);
