@@ -73,6 +73,8 @@ inline int per_device_value(std::atomic<int> (&cache)[kMaxDevices], F&& compute)
 // Programmatic dependent launch: a kernel launched with launch_dependent may become resident while
 // the kernel before it in the stream still runs, so it must pass dependency_wait (which holds until
 // that kernel has completed and its writes are visible) before it touches global memory.
+// Its pointer parameters carry no __restrict__ and it loads nothing through __ldg: what both promise is
+// read-only for the kernel's whole lifetime, which here begins while its predecessor still writes.
 // release_dependents lets the next such kernel start its launch; placed after the main work, so that
 // waiting CTAs do not hold SMs that other streams could use.
 // A solve is a chain of about a thousand launches of 4 to 50 us; the launch itself then overlaps the
@@ -116,6 +118,49 @@ ZDEV void for_entries(int m, int n, F&& f) {
     if (i >= m) {
       i -= m;
       ++j;
+    }
+  }
+}
+
+// for_entries in batches: v = f(i, j) for up to four entries of this thread, all loads in flight together, then
+// store(i, j, v) for them in the same order (after a store the compiler may not move the next load
+// up: it could read what was stored).  With __restrict__ and for_entries instead, which dependent kernels
+// may not use, 8192^2 took 411 us in combine_kernel (255 here), 147 in frob2_kernel (102), 260 in
+// copy_upper_kernel (211), 351 in scale_copy_kernel (358).  A store under a condition or one entry a
+// thread is better off with for_entries (shift_lower_kernel of eight 2048^2: 38 us, 49 here).
+template <class F, class G>
+ZDEV void map_entries(int m, int n, F&& f, G&& store) {
+  if (m <= 0) return;
+  constexpr int U = 4;
+  const unsigned stride = gridDim.x * blockDim.x, e0 = blockIdx.x * blockDim.x + threadIdx.x;
+  const int di = static_cast<int>(stride % m), dj = static_cast<int>(stride / m);
+  int i = static_cast<int>(e0 % m), j = static_cast<int>(e0 / m);
+  while (j < n) {
+    int vi[U], vj[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      vi[u] = i;
+      vj[u] = j;
+      i += di;
+      j += dj;
+      if (i >= m) {
+        i -= m;
+        ++j;
+      }
+    }
+    decltype(f(0, 0)) v[U];
+    if (vj[U - 1] < n) {  // all of them inside
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = f(vi[u], vj[u]);
+#pragma unroll
+      for (int u = 0; u < U; ++u) store(vi[u], vj[u], v[u]);
+    } else {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (vj[u] < n) v[u] = f(vi[u], vj[u]);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (vj[u] < n) store(vi[u], vj[u], v[u]);
     }
   }
 }

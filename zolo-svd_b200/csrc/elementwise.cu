@@ -19,7 +19,7 @@ inline int grid_for(int64_t work, int per_block = TPB) {
   return static_cast<int>(std::max<int64_t>(b, 1));
 }
 
-__global__ void scale_copy_kernel(int m, int n, double s, const double* __restrict__ src, int64_t lds,
+__global__ void scale_copy_kernel(int m, int n, double s, const double* src, int64_t lds,
                                   int64_t strideS, double* dst, int64_t ldd, int64_t strideD,
                                   double diag_add, const double* norm2) {
   dependency_wait();
@@ -28,14 +28,16 @@ __global__ void scale_copy_kernel(int m, int n, double s, const double* __restri
   const double* S = src + b * strideS;
   double* D = dst + b * strideD;
   if (norm2) s = 1.0 / sqrt(*norm2);
-  for_entries(m, n, [&](int i, int j) {
-    double v = s * S[i + j * lds];
-    if (i == j) v += diag_add;
-    D[i + j * ldd] = v;
-  });
+  map_entries(
+      m, n,
+      [&](int i, int j) {
+        const double v = s * S[i + j * lds];
+        return i == j ? v + diag_add : v;
+      },
+      [&](int i, int j, double v) { D[i + j * ldd] = v; });
 }
 
-__global__ void form_stack_kernel(int m, int mpad, int n, const double* __restrict__ X, int64_t ldx, double* W,
+__global__ void form_stack_kernel(int m, int mpad, int n, const double* X, int64_t ldx, double* W,
                                   int64_t ldw, int64_t strideW, const double* s_vec, double s_scalar,
                                   int x_upper, int64_t strideX) {
   dependency_wait();
@@ -45,15 +47,16 @@ __global__ void form_stack_kernel(int m, int mpad, int n, const double* __restri
   double* Wb = W + b * strideW;
   const double s = s_vec ? s_vec[b] : s_scalar;
   const int rows = mpad + n;
-  for_entries(rows, n, [&](int i, int j) {
-    double v;
-    if (i < m) v = (x_upper && i > j) ? 0.0 : X[i + j * ldx];
-    else v = (i - mpad == j) ? s : 0.0;
-    Wb[i + j * ldw] = v;
-  });
+  map_entries(
+      rows, n,
+      [&](int i, int j) {
+        if (i < m) return (x_upper && i > j) ? 0.0 : X[i + j * ldx];
+        return (i - mpad == j) ? s : 0.0;
+      },
+      [&](int i, int j, double v) { Wb[i + j * ldw] = v; });
 }
 
-__global__ void shift_lower_kernel(int n, const double* __restrict__ G, int64_t ldg, double* W,
+__global__ void shift_lower_kernel(int n, const double* G, int64_t ldg, double* W,
                                    int64_t ldw, int64_t strideW, const double* c_vec) {
   dependency_wait();
   release_dependents();
@@ -82,15 +85,12 @@ __device__ double block_sum(double v, double* sh) {
   return r;
 }
 
-__global__ void frob2_kernel(int m, int n, const double* __restrict__ X, int64_t ldx, double* partial) {
+__global__ void frob2_kernel(int m, int n, const double* X, int64_t ldx, double* partial) {
   dependency_wait();
   release_dependents();
   __shared__ double sh[TPB / 32];
   double s = 0.0;
-  for_entries(m, n, [&](int i, int j) {
-    const double v = X[i + j * ldx];
-    s += v * v;
-  });
+  map_entries(m, n, [&](int i, int j) { return X[i + j * ldx]; }, [&](int, int, double v) { s += v * v; });
   s = block_sum<TPB>(s, sh);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
@@ -105,7 +105,7 @@ __global__ void reduce_sum_kernel(const double* partial, int count, double* out)
   if (threadIdx.x == 0) out[0] = s;
 }
 
-__global__ void colsum_abs_kernel(int m, int n, const double* __restrict__ X, int64_t ldx, double* colsum) {
+__global__ void colsum_abs_kernel(int m, int n, const double* X, int64_t ldx, double* colsum) {
   dependency_wait();
   release_dependents();
   __shared__ double sh[TPB / 32];
@@ -133,27 +133,33 @@ __global__ void max_kernel(const double* v, int count, double* out) {
 }
 
 // X_new = cx*X + cz*sum_q Z_q ; partial = ||X_new - X||^2 per block.  In place on X.
-__global__ void combine_kernel(int m, int n, double* X, int64_t ldx, const double* __restrict__ Z,
+__global__ void combine_kernel(int m, int n, double* X, int64_t ldx, const double* Z,
                                int64_t ldz, int64_t strideZ, int nz, double cx, double cz,
-                               const double* __restrict__ cz_vec, double* partial) {
+                               const double* cz_vec, double* partial) {
   dependency_wait();
   release_dependents();
   __shared__ double sh[TPB / 32];
   double s = 0.0;
-  for_entries(m, n, [&](int i, int j) {
-    const double x = X[i + j * ldx];
-    double z = 0.0;
-    if (cz_vec) {
-      for (int q = 0; q < nz; ++q) z += cz_vec[q] * Z[q * strideZ + i + j * ldz];
-    } else {
-      for (int q = 0; q < nz; ++q) z += Z[q * strideZ + i + j * ldz];
-      z *= cz;
-    }
-    const double xn = cx * x + z;
+  auto update = [&](int i, int j, double x, double z) {
+    const double xn = cx * x + (cz_vec ? z : z * cz);
     const double d = x - xn;
     s += d * d;
     X[i + j * ldx] = xn;
-  });
+  };
+  if (nz == 1) {
+    const double w = cz_vec ? cz_vec[0] : 1.0;
+    map_entries(
+        m, n, [&](int i, int j) { return make_double2(X[i + j * ldx], 0.0 + w * Z[i + j * ldz]); },
+        [&](int i, int j, double2 v) { update(i, j, v.x, v.y); });
+  } else {
+    // several Z are already as many loads in flight
+    for_entries(m, n, [&](int i, int j) {
+      const double x = X[i + j * ldx];
+      double z = 0.0;
+      for (int q = 0; q < nz; ++q) z += (cz_vec ? cz_vec[q] : 1.0) * Z[q * strideZ + i + j * ldz];
+      update(i, j, x, z);
+    });
+  }
   s = block_sum<TPB>(s, sh);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
@@ -170,7 +176,7 @@ __global__ void symmetrize_kernel(int n, double* B, int64_t ldb) {
   });
 }
 
-__global__ void transpose_kernel(int m, int n, const double* __restrict__ A, int64_t lda, double* B,
+__global__ void transpose_kernel(int m, int n, const double* A, int64_t lda, double* B,
                                  int64_t ldb) {
   dependency_wait();
   release_dependents();
@@ -218,13 +224,13 @@ __global__ void mirror_lower_kernel(int n, double* B, int64_t ldb) {
   });
 }
 
-__global__ void copy_upper_kernel(int n, const double* __restrict__ A, int64_t lda, double scale, double* B,
+__global__ void copy_upper_kernel(int n, const double* A, int64_t lda, double scale, double* B,
                                   int64_t ldb) {
   dependency_wait();
   release_dependents();
-  for_entries(n, n, [&](int i, int j) {
-    B[i + static_cast<int64_t>(j) * ldb] = (i <= j) ? scale * A[i + static_cast<int64_t>(j) * lda] : 0.0;
-  });
+  map_entries(
+      n, n, [&](int i, int j) { return (i <= j) ? scale * A[i + static_cast<int64_t>(j) * lda] : 0.0; },
+      [&](int i, int j, double v) { B[i + static_cast<int64_t>(j) * ldb] = v; });
 }
 
 __global__ void set_identity_kernel(int m, int n, double* Q, int64_t ldq, int64_t strideQ, double diag) {

@@ -686,7 +686,7 @@ __global__ void __launch_bounds__(NW * 32, 1) qr_panel_reg_kernel(PanelArgs p) {
   }
 }
 
-__global__ void extract_v_kernel(int m, int w, const double* __restrict__ A, int64_t lda, int64_t strideA,
+__global__ void extract_v_kernel(int m, int w, const double* A, int64_t lda, int64_t strideA,
                                  double* V, int64_t ldv, int64_t strideV, int split, int64_t gap) {
   dependency_wait();
   release_dependents();
