@@ -204,6 +204,12 @@ int zolo_profile_read(zolo_handle_t handle, double* out, int reset);
  * smaller nodes use QDWH, those of one recursion level as one batched solve; 0 = QDWH for
  * every node (pqdwhsubit.f90's polar factor).  The later candidate shifts always use QDWH. */
 #define ZOLO_OPT_EIG_ZOLO_MIN 13
+/* ZOLO_OPT_PANEL_WAIT (diagnostic): limit, in clock cycles of an SM, of the waits between the
+ * thread blocks of a Householder panel; 0 (default) = 2e9, about a second; -1 = every such wait
+ * has run out.  A panel whose wait runs out is given up and its call returns -2911 (-2912 when
+ * the messages between its blocks did not arrive within the default limit either): the
+ * results of that call are not to be used, the handle stays usable. */
+#define ZOLO_OPT_PANEL_WAIT 14
 /* The default handle (used by the reference-named host-array entry points) reads its options
  * from the environment when it is created, so an unchanged Fortran driver selects them:
  * ZOLO_FAST=1 sets ZOLO_OPT_SHARED_QR, _NS_FINISH, _CHOL_INVERSE, _BETA_FROB, _TERM_PLAN and

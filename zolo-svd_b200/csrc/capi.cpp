@@ -150,6 +150,15 @@ int set_option(Context& c, int option, int value) {
       if (value < 0) return -3;
       c.eig_zolo_min = value;
       return 0;
+    case ZOLO_OPT_PANEL_WAIT:
+      if (value < -1) return -3;
+      if (value != c.panel_wait) {  // captured launches hold the limit
+        c.sync_all();
+        c.drop_graphs();
+        for (auto& w : c.workers) w->drop_graphs();
+      }
+      c.panel_wait = value;
+      return 0;
     default:
       return -1;
   }
@@ -353,6 +362,7 @@ int zolo_get_option(zolo_handle_t h, int option, int* value) {
       case ZOLO_OPT_BATCH_GRAPH: *value = c.batch_graph; return 0;
       case ZOLO_OPT_INJECT_BATCH_ERR: *value = c.inject_batch_err; return 0;
       case ZOLO_OPT_EIG_ZOLO_MIN: *value = c.eig_zolo_min; return 0;
+      case ZOLO_OPT_PANEL_WAIT: *value = c.panel_wait; return 0;
       default: return -1;
     }
   });

@@ -118,6 +118,9 @@ class Context {
   // diagnostic: 1 = the batched solver's scheduled run sees its first member's last error
   // above the stopping tolerance (0 = off)
   int inject_batch_err = 0;
+  // diagnostic: limit of the waits between the CTAs of a Householder panel in clock cycles, 0 = the
+  // kernel's own, -1 = every one of them has run out
+  int panel_wait = 0;
   // eigensolver: nodes of at least this size split with the Zolo-PD fast form (r = 8, every
   // cost option), smaller ones with QDWH (batched per level); 0 = QDWH for every node
   int eig_zolo_min = 4096;

@@ -144,6 +144,7 @@ void run_concurrent(Context& c, int count, const std::vector<double>& cost, F&& 
         wc.zolo_mixed = c.zolo_mixed;
         wc.oz_slices = c.oz_slices;
         wc.eig_zolo_min = c.eig_zolo_min;
+        wc.panel_wait = c.panel_wait;
         for (int i : assign[w]) {
           if (stop) break;
           task(wc, i);

@@ -131,10 +131,13 @@ cudaError_t trtri_blocks(int n, const double* L, int64_t ldl, int64_t strideL, d
 // of the compact WY form I - V T V^T.  Vexp receives V explicitly (m x w, ldv).
 // Row gap: with split > 0, logical row r >= split of the panel is the physical
 // row r + gap of A (two row segments; Vexp stays in logical rows).  Vexp may be null up to 8192 rows.
+// status (in mapped host memory): 911 when a wait between the CTAs of a cluster ran out, 912 when
+// its messages in flight did not arrive afterwards either; the panel is then not factored.  wait_limit: clock
+// cycles of such a wait, 0 = 2e9, below zero = none.
 cudaError_t qr_panel(int m, int w, double* A, int64_t lda, int64_t strideA, double* tau,
                      int64_t strideTau, double* T, int64_t strideT, double* Vexp, int64_t ldv,
                      int64_t strideV, int batch, cudaStream_t st, int split = 0, int64_t gap = 0,
-                     int* status = nullptr);
+                     int* status = nullptr, long long wait_limit = 0);
 // Cluster size the panel kernel uses for an m x w panel (negative: rows stay in global memory).
 int qr_panel_config(int m, int w);
 // Vexp = unit-lower-trapezoidal V taken from A (m x w logical rows, same row gap

@@ -416,7 +416,7 @@ static void factor_panel(Context& c, int mtot, int n, int m_top, bool top_tri, i
   Profiler::Rec rec;
   if (c.prof.on) c.prof.begin(1, 2.0 * R.mp * static_cast<double>(jb) * jb * batch, st, &rec);
   ck(qr_panel(R.mp, jb, W.at(j, j).p, W.ld, W.stride, tau + j, n, T + (j / PW) * PW * PW, strideT, Vp.p, Vp.ld,
-              Vp.stride, batch, st, R.split, R.gap, c.fault_word()));
+              Vp.stride, batch, st, R.split, R.gap, c.fault_word(), c.panel_wait));
   if (c.prof.on) c.prof.end(rec, st);
   c.stats.launches++;
 }

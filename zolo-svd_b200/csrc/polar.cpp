@@ -1333,6 +1333,7 @@ int qdwh_batch(Context& c, int count, const int* m, const int* n, const double* 
           wc.batch_graph = c.batch_graph;
           wc.inject_chol_fail = c.inject_chol_fail;
           wc.inject_batch_err = c.inject_batch_err;
+          wc.panel_wait = c.panel_wait;
           for (int b : assign[w])
             qdwh_bucket(wc, plan.members[b], plan.mb[b], plan.nb[b], m, n, dA, lda, dQ, ldq, dH, ldh, info,
                         iterations, &wbs[w]);
@@ -1387,6 +1388,7 @@ int batch_autotune(Context& c) {
   wc.batch_graph = c.batch_graph;
   wc.inject_chol_fail = 0;
   wc.inject_batch_err = 0;
+  wc.panel_wait = c.panel_wait;
   for (int k = 0; k < 3; ++k) {
     const int NB = sizes[k], MB = NB + NB / 2;
     std::vector<double> host(static_cast<size_t>(MB) * NB, 0.0);

@@ -58,7 +58,8 @@ struct PanelArgs {
   int64_t strideT;
   double* V;
   int64_t ldv, strideV;
-  int* status;  // written when a wait between the CTAs timed out
+  int* status;           // written when a wait between the CTAs timed out
+  long long wait_limit;  // clock cycles of such a wait
 };
 
 ZDEV double group_sum8(double v) {
@@ -392,7 +393,7 @@ struct RegShared {
   double T[QW][QW];         // T[j][i] = T(i, j)
   unsigned long long bar[2];
   uint32_t peer[QCL];  // shared-window addresses of this struct in the other CTAs, own CTA first
-  int abort;
+  int abort;  // 1 + the column at which this CTA's wait ran out, 0 = none
 };
 
 ZDEV uint32_t cluster_addr(const void* p, int rank) {
@@ -410,9 +411,12 @@ ZDEV void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 constexpr long long kPanelTimeoutCycles = 2000000000LL;  // about a second
-// Bounded wait of one warp on its CTA's mbarrier phase.
-ZDEV bool panel_wait(uint32_t bar, uint32_t parity) {
+// Wait of one warp on its CTA's mbarrier phase for at most `limit` clock cycles, not at all below
+// zero; a last look follows the limit, for a GPU that was switched away meanwhile.
+ZDEV bool panel_wait(uint32_t bar, uint32_t parity, long long limit) {
+  if (limit < 0) return false;
   const long long t0 = clock64();
+  bool late = false;
   while (true) {
     uint32_t ok;
     asm volatile(
@@ -423,7 +427,8 @@ ZDEV bool panel_wait(uint32_t bar, uint32_t parity) {
         : "r"(bar), "r"(parity)
         : "memory");
     if (ok) return true;
-    if (clock64() - t0 > kPanelTimeoutCycles) return false;
+    if (late) return false;
+    late = clock64() - t0 > limit;
   }
 }
 
@@ -448,6 +453,21 @@ ZDEV void panel_send(Sh& S, const void* slot, const void* bar, double v, bool al
   }
 }
 
+// This CTA's sums of column k: columns c >= k to every CTA, c < k to the last one only (the pivot row
+// goes by itself), and what column k will bring to this CTA armed on its barrier; one warp.
+template <class Sh>
+ZDEV void panel_send_sums(Sh& S, int k, double sum, int rank, int CL) {
+  const int lane = threadIdx.x & 31, buf = k & 1;
+  if (lane == 0) {
+    const int bytes = (rank == CL - 1 ? QW : QW - k) * 8 * CL + QW * 8;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(&S.bar[buf]))),
+                 "r"(bytes)
+                 : "memory");
+  }
+  panel_send(S, &S.recv[buf][rank][lane], &S.bar[buf], sum, lane >= k, rank, CL);
+}
+
 // Column k of T by one warp (dlarft, forward, columnwise): T(k,k) = tau_k,
 // T(i,k) = -tau_k sum_{i <= j < k} T(i,j) v_j^T v_k; lane i forms row i.
 ZDEV void panel_t_column(double (*T)[QW], const double* z, double tau, int k) {
@@ -467,7 +487,8 @@ ZDEV void panel_t_column(double (*T)[QW], const double* z, double tau, int k) {
 // at or past nloc hold zeros).  On return (all warps past a CTA barrier) S.tau is complete in
 // every CTA and S.T in the last one.  False after a timed-out wait.
 template <int NW, int RN>
-ZDEV bool panel_factor(double (&a)[RN][8], RegShared<NW>& S, int w, int r0, int nloc, int rank, int CL) {
+ZDEV bool panel_factor(double (&a)[RN][8], RegShared<NW>& S, int w, int r0, int nloc, int rank, int CL,
+                       long long wait_limit) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int rbase = r0 + warp * 8 * RN + g;  // global row of a[0]
   // the column whose warp sum ends in this lane after the halving stages
@@ -533,14 +554,8 @@ ZDEV bool panel_factor(double (&a)[RN][8], RegShared<NW>& S, int w, int r0, int 
           double sum = (s4[0] + s4[1]) + (s4[2] + s4[3]), pr;
           if (CL > 1) {
             const uint32_t bar = bar0 + 8 * buf;
-            // columns c >= k to every CTA, c < k to the last one only; the pivot row by warp 1
-            if (lane == 0) {
-              const int bytes = (last ? QW : QW - k) * 8 * CL + QW * 8;
-              asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-                           : "memory");
-            }
-            panel_send(S, &S.recv[buf][rank][lane], &S.bar[buf], sum, lane >= k, rank, CL);
-            if (!panel_wait(bar, (k >> 1) & 1)) S.abort = 1;
+            panel_send_sums(S, k, sum, rank, CL);
+            if (!panel_wait(bar, (k >> 1) & 1, wait_limit)) S.abort = k + 1;
 #pragma unroll
             for (int q = 0; q < 4; ++q) s4[q] = 0.0;
 #pragma unroll
@@ -614,6 +629,40 @@ done:
   return true;
 }
 
+// After a wait of this CTA ran out at column k = S.abort - 1, before it may leave (all threads): what the
+// others sent to it is on its way (st.async is not ordered by the cluster barrier) and must not arrive
+// in shared memory that is no longer its own.  A CTA sends column k + 1 only after all of column k
+// has reached it, so the CTAs that give up stand at one column or at two neighbouring ones:
+// those behind send the next column too, and every phase then completes.  A CTA that gives up before the
+// last column keeps all others from finishing, so all of them come here; after the last column
+// others may have left, but then nothing is missing and nothing of theirs is read.  False when the phases
+// did not complete in time either.
+template <int NW>
+ZDEV bool panel_drain(RegShared<NW>& S, int w, int r0, int nloc, int rank, int CL) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int k = S.abort - 1;
+  int top = k;
+  __syncwarp();
+  cluster_sync_all();  // every CTA that gave up has written its column
+  if (k < w - 1) {
+    cg::cluster_group cluster = cg::this_cluster();
+    for (int q = 0; q < CL; ++q) top = max(top, *cluster.map_shared_rank(&S.abort, q) - 1);
+  }
+  bool ok = true;
+  if (top > k && warp == 1 && top >= r0 && top < r0 + nloc)
+    panel_send(S, &S.prow_in[top & 1][lane], &S.bar[top & 1], 0.0, true, rank, CL);
+  if (warp == 0) {
+    if (top > k) panel_send_sums(S, top, 0.0, rank, CL);
+    for (int c = max(top - 1, 0); c <= top; ++c)
+      ok = panel_wait(static_cast<uint32_t>(__cvta_generic_to_shared(&S.bar[c & 1])), (c >> 1) & 1,
+                      kPanelTimeoutCycles) &&
+           ok;
+  }
+  __syncwarp();
+  cluster_sync_all();  // no CTA leaves while another reads its column
+  return ok;
+}
+
 template <int NW, int RN>
 __global__ void __launch_bounds__(NW * 32, 1) qr_panel_reg_kernel(PanelArgs p) {
   __shared__ __align__(16) RegShared<NW> S;
@@ -653,12 +702,12 @@ __global__ void __launch_bounds__(NW * 32, 1) qr_panel_reg_kernel(PanelArgs p) {
 #pragma unroll
     for (int i = 0; i < RN; ++i) a[i][j] = (in && l0 + 8 * i < nloc) ? col[ro[i]] : 0.0;
   }
-  if (!panel_factor<NW, RN>(a, S, w, r0, nloc, rank, CL)) {
+  if (!panel_factor<NW, RN>(a, S, w, r0, nloc, rank, CL, p.wait_limit)) {
+    const bool drained = panel_drain(S, w, r0, nloc, rank, CL);
     if (threadIdx.x == 0 && p.status) {
-      *static_cast<volatile int*>(p.status) = 911;
+      *static_cast<volatile int*>(p.status) = drained ? 911 : 912;
       __threadfence_system();
     }
-    cluster_sync_all();  // no CTA leaves while others may still send to it
     return;
   }
   release_dependents();
@@ -945,7 +994,7 @@ int qr_panel_config(int m, int w) {
 
 cudaError_t qr_panel(int m, int w, double* A, int64_t lda, int64_t strideA, double* tau, int64_t strideTau,
                      double* T, int64_t strideT, double* Vexp, int64_t ldv, int64_t strideV, int batch,
-                     cudaStream_t st, int split, int64_t gap, int* status) {
+                     cudaStream_t st, int split, int64_t gap, int* status, long long wait_limit) {
   if (m <= 0 || w <= 0 || batch <= 0) return cudaSuccess;
   if (w > QW || m < w || gap < 0 || (gap > 0 && split < w)) return cudaErrorInvalidValue;
   const int maxcl = max_cluster();
@@ -972,6 +1021,7 @@ cudaError_t qr_panel(int m, int w, double* A, int64_t lda, int64_t strideA, doub
   pa.ldv = ldv;
   pa.strideV = strideV;
   pa.status = status;
+  pa.wait_limit = wait_limit == 0 ? kPanelTimeoutCycles : wait_limit;
   int rcl = 0, rnw = 0;
   if (reg_config(m, batch, maxcl, &rcl, &rnw)) {
     pa.rows_per = (m + rcl - 1) / rcl;
