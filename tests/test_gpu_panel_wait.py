@@ -95,3 +95,20 @@ def test_option_values(h):
     assert zb.lib().zolo_set_option(h.ptr, zb.OPT_PANEL_WAIT, -2) == -3
     h.set_option(zb.OPT_PANEL_WAIT, -1)
     assert h.get_option(zb.OPT_PANEL_WAIT) == -1
+
+
+def test_code_is_not_left_for_the_next_call(h):
+    """A call in which a wait ran out and which then ends with another error keeps its code to itself."""
+    import torch
+    m, n = 700, 64
+    dx = zb.colmajor_to_device(np.random.default_rng(2).standard_normal((m, n)))
+    dz = torch.zeros((n, m + 2), dtype=torch.float64, device="cuda")
+
+    def zoloqr(ptr):
+        return zb.lib().zolo_zoloqr_dev(h.ptr, m, n, dx.data_ptr(), m, 0.5, 1.0, ptr, m + 2)
+
+    h.set_option(zb.OPT_PANEL_WAIT, -1)
+    # Z off an 8-byte boundary: refused on the host (716) at the last product, after the panels
+    assert zoloqr(dz.data_ptr() + 4) == -1716
+    h.set_option(zb.OPT_PANEL_WAIT, 0)
+    assert zoloqr(dz.data_ptr()) == 0

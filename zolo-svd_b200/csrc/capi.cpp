@@ -57,8 +57,10 @@ int guarded(zolo_handle_t h, F&& f) {
     if (const int fault = h->ctx.take_fault()) return r < 0 ? r : kWaitBase - fault;
     return r;
   } catch (const CudaFailure& e) {
+    h->ctx.settle();
     return kCudaBase - static_cast<int>(e.err);
   } catch (const std::bad_alloc&) {
+    h->ctx.settle();
     return kCudaBase - static_cast<int>(cudaErrorMemoryAllocation);
   }
 }

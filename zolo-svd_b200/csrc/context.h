@@ -173,6 +173,12 @@ class Context {
   // the first fault code of this context and its workers since the last call (cleared), 0 = none;
   // complete once the streams have been synchronized
   int take_fault();
+  // after a call that ended with an error: waits for what it queued and drops its fault code, which is
+  // not the next call's
+  void settle() {
+    sync_all();
+    take_fault();
+  }
 
  private:
   int device_;
