@@ -130,7 +130,8 @@ cudaError_t trtri_blocks(int n, const double* L, int64_t ldl, int64_t strideL, d
 // diagonal (unit diagonal implied), R on/above it, tau[w], T (w x w upper, ld 32)
 // of the compact WY form I - V T V^T.  Vexp receives V explicitly (m x w, ldv).
 // Row gap: with split > 0, logical row r >= split of the panel is the physical
-// row r + gap of A (two row segments; Vexp stays in logical rows).  Vexp may be null up to 8192 rows.
+// row r + gap of A (two row segments; Vexp stays in logical rows).  Vexp may be null for a panel that fits the
+// registers of one cluster: up to 512 panel_cluster_max() rows, 8192 with clusters of 16.
 // status (in mapped host memory): 911 when a wait between the CTAs of a cluster ran out, 912 when
 // its messages in flight did not arrive afterwards either; the panel is then not factored.  wait_limit: clock
 // cycles of such a wait, 0 = 2e9, below zero = none.

@@ -1031,6 +1031,7 @@ cudaError_t qr_panel(int m, int w, double* A, int64_t lda, int64_t strideA, doub
       default: return launch_reg<16, 4>(pa, rcl, batch, st);
     }
   }
+  if (!Vexp) return cudaErrorInvalidValue;  // the panels below always write V
   const size_t chunk = static_cast<size_t>(pa.rp_ld) * w * 8;
   if (chunk <= SMEM_CHUNK_CAP) return launch_panel<true>(pa, cl, batch, shared_base() + chunk, st);
   return launch_panel<false>(pa, cl, batch, shared_base(), st);
