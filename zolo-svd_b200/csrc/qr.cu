@@ -580,6 +580,7 @@ ZDEV bool panel_factor(double (&a)[RN][8], RegShared<NW>& S, int w, int r0, int 
             // chain is 150 clocks longer
             const double z = alpha - beta;
             scal = copysign(rsqrt(z * z), z);
+            if (n2 > 0x1p1021) scal = 1.0 / z;  // |z| is up to twice the norm: z^2 may pass the largest number
             tau = (beta - alpha) * rb;
           }
           const double vta = fma(scal, sum, pr);
