@@ -411,10 +411,9 @@ ZDEV void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 constexpr long long kPanelTimeoutCycles = 2000000000LL;  // about a second
-// Wait of one warp on its CTA's mbarrier phase for at most `limit` clock cycles, not at all below
-// zero; a last look follows the limit, for a GPU that was switched away meanwhile.
+// Wait of one warp on its CTA's mbarrier phase for at most `limit` clock cycles (below zero: it has run
+// out whatever comes); a last look follows the limit, for a GPU that was switched away meanwhile.
 ZDEV bool panel_wait(uint32_t bar, uint32_t parity, long long limit) {
-  if (limit < 0) return false;
   const long long t0 = clock64();
   bool late = false;
   while (true) {
@@ -426,7 +425,7 @@ ZDEV bool panel_wait(uint32_t bar, uint32_t parity, long long limit) {
         : "=r"(ok)
         : "r"(bar), "r"(parity)
         : "memory");
-    if (ok) return true;
+    if (ok && limit >= 0) return true;
     if (late) return false;
     late = clock64() - t0 > limit;
   }
@@ -456,14 +455,11 @@ ZDEV void panel_send(Sh& S, const void* slot, const void* bar, double v, bool al
 // This CTA's sums of column k: columns c >= k to every CTA, c < k to the last one only (the pivot row
 // goes by itself), and what column k will bring to this CTA armed on its barrier; one warp.
 template <class Sh>
-ZDEV void panel_send_sums(Sh& S, int k, double sum, int rank, int CL) {
-  const int lane = threadIdx.x & 31, buf = k & 1;
+ZDEV void panel_send_sums(Sh& S, uint32_t bar, int k, int buf, double sum, int rank, int CL) {
+  const int lane = threadIdx.x & 31;
   if (lane == 0) {
     const int bytes = (rank == CL - 1 ? QW : QW - k) * 8 * CL + QW * 8;
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
-                     static_cast<uint32_t>(__cvta_generic_to_shared(&S.bar[buf]))),
-                 "r"(bytes)
-                 : "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
   }
   panel_send(S, &S.recv[buf][rank][lane], &S.bar[buf], sum, lane >= k, rank, CL);
 }
@@ -554,7 +550,7 @@ ZDEV bool panel_factor(double (&a)[RN][8], RegShared<NW>& S, int w, int r0, int 
           double sum = (s4[0] + s4[1]) + (s4[2] + s4[3]), pr;
           if (CL > 1) {
             const uint32_t bar = bar0 + 8 * buf;
-            panel_send_sums(S, k, sum, rank, CL);
+            panel_send_sums(S, bar, k, buf, sum, rank, CL);
             if (!panel_wait(bar, (k >> 1) & 1, wait_limit)) S.abort = k + 1;
 #pragma unroll
             for (int q = 0; q < 4; ++q) s4[q] = 0.0;
@@ -568,7 +564,7 @@ ZDEV bool panel_factor(double (&a)[RN][8], RegShared<NW>& S, int w, int r0, int 
           }
           const double s0 = __shfl_sync(0xffffffffu, sum, k);
           const double alpha = __shfl_sync(0xffffffffu, pr, k);
-          double beta = alpha, tau = 0.0, scal = 0.0, rb = 0.0;
+          double beta = alpha, tau = 0.0, rb = 0.0, rz = 0.0, half = 1.0;
           if (s0 != 0.0) {
             // norm and its reciprocal from one rsqrt (norm corrected by a Newton step)
             const double n2 = fma(alpha, alpha, s0), r = rsqrt(n2);
@@ -577,17 +573,18 @@ ZDEV bool panel_factor(double (&a)[RN][8], RegShared<NW>& S, int w, int r0, int 
             beta = -copysign(nrm, alpha);
             rb = -copysign(r, alpha);
             // 1/(alpha - beta), its magnitude |alpha| + norm >= norm, as rsqrt of its square: a division's
-            // chain is 150 clocks longer
-            const double z = alpha - beta;
-            scal = copysign(rsqrt(z * z), z);
-            if (n2 > 0x1p1021) scal = 1.0 / z;  // |z| is up to twice the norm: z^2 may pass the largest number
+            // chain is 150 clocks longer.  Of half of it where the square of up to twice the norm may
+            // pass the largest number (n2 >= 2^1021); a branch to a division there cost 36 clocks.
+            half = __double2hiint(n2) >= 0x7fc00000 ? 0.5 : 1.0;
+            const double z = fma(half, nrm, half * fabs(alpha));
+            rz = copysign(rsqrt(z * z), alpha);
             tau = (beta - alpha) * rb;
           }
-          const double vta = fma(scal, sum, pr);
+          const double vta = fma(rz, half * sum, pr);
           S.w[lane] = lane > k ? vta * rb : 0.0;
           S.Z[buf][lane] = vta;
           if (lane == 0) {
-            S.sc[0] = scal;
+            S.sc[0] = half * rz;
             S.sc[1] = beta;
             S.sc[2] = alpha - beta;
             S.tau[k] = tau;
@@ -653,11 +650,10 @@ ZDEV bool panel_drain(RegShared<NW>& S, int w, int r0, int nloc, int rank, int C
   if (top > k && warp == 1 && top >= r0 && top < r0 + nloc)
     panel_send(S, &S.prow_in[top & 1][lane], &S.bar[top & 1], 0.0, true, rank, CL);
   if (warp == 0) {
-    if (top > k) panel_send_sums(S, top, 0.0, rank, CL);
+    const uint32_t bar0 = static_cast<uint32_t>(__cvta_generic_to_shared(&S.bar[0]));
+    if (top > k) panel_send_sums(S, bar0 + 8 * (top & 1), top, top & 1, 0.0, rank, CL);
     for (int c = max(top - 1, 0); c <= top; ++c)
-      ok = panel_wait(static_cast<uint32_t>(__cvta_generic_to_shared(&S.bar[c & 1])), (c >> 1) & 1,
-                      kPanelTimeoutCycles) &&
-           ok;
+      ok = panel_wait(bar0 + 8 * (c & 1), (c >> 1) & 1, kPanelTimeoutCycles) && ok;
   }
   __syncwarp();
   cluster_sync_all();  // no CTA leaves while another reads its column
