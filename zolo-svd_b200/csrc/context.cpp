@@ -15,13 +15,13 @@ Context::Context(int device) : device_(device) {
   ck(cudaStreamCreateWithPriority(&side_, cudaStreamDefault, hi));
   for (auto& e : ev_) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   void* f = nullptr;
-  ck(cudaHostAlloc(&f, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
-  fault_ = static_cast<int*>(f);  // one address for host and device (unified addressing)
-  *fault_ = 0;
+  ck(cudaHostAlloc(&f, sizeof(HostWords), cudaHostAllocMapped | cudaHostAllocPortable));
+  host_ = static_cast<HostWords*>(f);  // one address for host and device (unified addressing)
+  *host_ = HostWords{0, 0.0};
 }
 
 int Context::take_fault() {
-  volatile int* f = fault_;
+  volatile int* f = &host_->fault;
   int code = *f;
   if (code) *f = 0;
   for (auto& w : workers) {
@@ -37,7 +37,7 @@ Context::~Context() {
     if (e) cudaEventDestroy(e);
   if (side_) cudaStreamDestroy(side_);
   if (own_stream_) cudaStreamDestroy(own_stream_);
-  if (fault_) cudaFreeHost(fault_);
+  if (host_) cudaFreeHost(host_);
 }
 
 void Context::drop_graphs() {

@@ -169,7 +169,9 @@ class Context {
   int* dinfo();        // 1024 ints
   int* oz_status_word();  // status of the INT8-emulated products (zeroed when allocated)
   // word in mapped host memory that a kernel writes when one of its bounded waits timed out
-  int* fault_word() { return fault_; }
+  int* fault_word() { return &host_->fault; }
+  // ||A||_F^2 of the bounds in mapped host memory, written by the GPU as soon as it is known
+  volatile double* norm_word() { return &host_->norm2; }
   // the first fault code of this context and its workers since the last call (cleared), 0 = none;
   // complete once the streams have been synchronized
   int take_fault();
@@ -189,7 +191,11 @@ class Context {
   std::multimap<size_t, void*> pool_;
   std::mutex pool_mu_;
   uint64_t alloc_gen_ = 0;
-  int* fault_ = nullptr;
+  struct HostWords {  // mapped host memory
+    int fault;
+    double norm2;
+  };
+  HostWords* host_ = nullptr;
   void* grow(const std::string& name, size_t bytes);
 };
 

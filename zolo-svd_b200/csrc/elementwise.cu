@@ -21,13 +21,19 @@ inline int grid_for(int64_t work, int per_block = TPB) {
 
 __global__ void scale_copy_kernel(int m, int n, double s, const double* src, int64_t lds,
                                   int64_t strideS, double* dst, int64_t ldd, int64_t strideD,
-                                  double diag_add, const double* norm2) {
+                                  double diag_add, const double* norm2, volatile double* host) {
   dependency_wait();
   release_dependents();
   const int b = blockIdx.y;
   const double* S = src + b * strideS;
   double* D = dst + b * strideD;
-  if (norm2) s = 1.0 / sqrt(*norm2);
+  if (norm2) {
+    s = 1.0 / sqrt(*norm2);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      *host = *norm2;
+      __threadfence_system();
+    }
+  }
   map_entries(
       m, n,
       [&](int i, int j) {
@@ -312,13 +318,14 @@ cudaError_t get_diag(int n, const double* A, int64_t lda, double* d, cudaStream_
 cudaError_t scale_copy(int m, int n, double s, const double* src, int64_t lds, int64_t strideS, double* dst,
                        int64_t ldd, int64_t strideD, int batch, double diag_add, cudaStream_t st) {
   if (m <= 0 || n <= 0 || batch <= 0) return cudaSuccess;
-  return launch_dependent(scale_copy_kernel, dim3(grid_for(static_cast<int64_t>(m) * n), batch), dim3(TPB), 0, st, dim3(1), m, n, s, src, lds, strideS, dst, ldd, strideD, diag_add, nullptr);
+  return launch_dependent(scale_copy_kernel, dim3(grid_for(static_cast<int64_t>(m) * n), batch), dim3(TPB), 0, st, dim3(1), m, n, s, src, lds, strideS, dst, ldd, strideD, diag_add, nullptr, nullptr);
 }
 
-cudaError_t scale_by_norm(int m, int n, const double* norm2, double* X, int64_t ldx, cudaStream_t st) {
+cudaError_t scale_by_norm(int m, int n, const double* norm2, double* X, int64_t ldx, volatile double* host,
+                          cudaStream_t st) {
   if (m <= 0 || n <= 0) return cudaSuccess;
   return launch_dependent(scale_copy_kernel, dim3(grid_for(static_cast<int64_t>(m) * n)), dim3(TPB), 0, st, dim3(1), m,
-                          n, 0.0, X, ldx, 0, X, ldx, 0, 0.0, norm2);
+                          n, 0.0, X, ldx, 0, X, ldx, 0, 0.0, norm2, host);
 }
 
 cudaError_t form_stack(int m, int mpad, int n, const double* X, int64_t ldx, double* W, int64_t ldw,

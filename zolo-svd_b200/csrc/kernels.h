@@ -66,8 +66,9 @@ cudaError_t ozgemm(const GemmArgs& a, int slices, const OzWork& w, cudaStream_t 
 cudaError_t scale_copy(int m, int n, double s, const double* src, int64_t lds, int64_t strideS,
                        double* dst, int64_t ldd, int64_t strideD, int batch, double diag_add,
                        cudaStream_t st);
-// X <- X / sqrt(*norm2), norm2 on the device
-cudaError_t scale_by_norm(int m, int n, const double* norm2, double* X, int64_t ldx, cudaStream_t st);
+// X <- X / sqrt(*norm2), norm2 on the device; its value also to *host (mapped host memory)
+cudaError_t scale_by_norm(int m, int n, const double* norm2, double* X, int64_t ldx, volatile double* host,
+                          cudaStream_t st);
 // W = [X; 0; s I]: X (m x n) in rows [0,m), zeros in [m,mpad), s I in rows [mpad, mpad+n)
 // (mpad >= m keeps the identity block at an even row offset), batched over s_vec[b] or s_scalar.
 // x_upper: take only the upper triangle of X (zeros below its diagonal).  strideX: X of

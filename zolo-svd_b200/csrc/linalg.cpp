@@ -424,8 +424,8 @@ static void factor_panel(Context& c, int mtot, int n, int m_top, bool top_tri, i
 // Householder QR panel by panel.  The chain (a panel, its reflector on the next panel's columns, the
 // next panel) runs on the high-priority side stream alone, so that no step of it waits for another
 // stream's event; the main stream updates the columns further right beside the next panel.
-static void geqrf_panelwise(Context& c, int mtot, int n, int m_top, Mat W, double* tau, double* T, int64_t strideT,
-                            int batch, bool top_tri) {
+static bool geqrf_panelwise(Context& c, int mtot, int n, int m_top, Mat W, double* tau, double* T, int64_t strideT,
+                            int batch, bool top_tri, const std::function<bool()>& keep_on) {
   cudaStream_t ms = c.stream(), ss = c.side_stream();
   const Mat none{nullptr, 0, 0};
   if (n <= 2 * PW) ss = ms;  // nothing to update beside a panel
@@ -434,10 +434,15 @@ static void geqrf_panelwise(Context& c, int mtot, int n, int m_top, Mat W, doubl
     ck(cudaStreamWaitEvent(ss, c.event(0), 0));
   }
   bool rest = false;  // an update of the main stream that the next step on the side stream needs
+  bool whole = true;
   for (int j = 0; j < n; j += PW) {
     factor_panel(c, mtot, n, m_top, top_tri, j, W, tau, T, strideT, none, batch, ss);
     const int nc = n - j - PW, jn = std::min(PW, nc);
     if (nc <= 0) break;
+    if (j == 0 && keep_on && !keep_on()) {
+      whole = false;
+      break;
+    }
     const PanelRows R = panel_rows(mtot, m_top, top_tri, j, PW);
     const double* Tj = T + (j / PW) * PW * PW;
     if (nc > jn) ck(cudaEventRecord(c.event(0), ss));
@@ -454,6 +459,7 @@ static void geqrf_panelwise(Context& c, int mtot, int n, int m_top, Mat W, doubl
     ck(cudaEventRecord(c.event(0), ss));
     ck(cudaStreamWaitEvent(ms, c.event(0), 0));
   }
+  return whole;
 }
 
 // Householder QR in 128-column blocks of four 32-column panels.  Inside a block each panel
@@ -461,11 +467,13 @@ static void geqrf_panelwise(Context& c, int mtot, int n, int m_top, Mat W, doubl
 // rank-128 update per block, C -= V_B (T_B^T (V_B^T C)), whose GEMMs have K = rows and
 // K = 128.  Look-ahead: the next block's columns are updated first, then the next block is
 // factored on the side stream while the main stream updates the rest.
-void geqrf(Context& c, int mtot, int n, int m_top, Mat W, double* tau, double* T, int batch, bool top_tri) {
+bool geqrf(Context& c, int mtot, int n, int m_top, Mat W, double* tau, double* T, int batch, bool top_tri,
+           const std::function<bool()>& keep_on) {
   const int npan = (n + PW - 1) / PW;
   const int64_t ldv = (mtot + 1) / 2 * 2;
   const int64_t strideT = static_cast<int64_t>(npan) * PW * PW;
-  if (panelwise(mtot, n, batch, true)) return geqrf_panelwise(c, mtot, n, m_top, W, tau, T, strideT, batch, top_tri);
+  if (panelwise(mtot, n, batch, true))
+    return geqrf_panelwise(c, mtot, n, m_top, W, tau, T, strideT, batch, top_tri, keep_on);
   Mat Vp{c.buf("qr_v2", static_cast<size_t>(ldv) * PW * batch), ldv, ldv * PW};
   Mat Pp{c.buf("qr_p", static_cast<size_t>(PW) * QB * batch), PW, static_cast<int64_t>(PW) * QB};
   Mat VB{c.buf("qr_vb", static_cast<size_t>(ldv) * QB * batch), ldv, ldv * QB};
@@ -484,6 +492,7 @@ void geqrf(Context& c, int mtot, int n, int m_top, Mat W, double* tau, double* T
       // least; a large batch is past latency, and the products' 10 TF/s beat its 4.6
       const bool one = reflect_applies(R.mp) && static_cast<double>(R.mp) * nc * batch <= 1.2e6;
       factor_panel(c, mtot, n, m_top, top_tri, j, W, tau, T, strideT, one ? Mat{nullptr, 0, 0} : Vp, batch, st);
+      if (j == 0 && n > PW && keep_on && !keep_on()) return false;
       if (nc <= 0) continue;
       if (one) {
         apply_panel(c, R, jb, nc, W.at(j, j), T + pj * PW * PW, strideT, 1, W.at(j, j + jb), batch, st);
@@ -494,8 +503,9 @@ void geqrf(Context& c, int mtot, int n, int m_top, Mat W, double* tau, double* T
       c.stats.launches++;
       panel_b_minus_vp(c, R, jb, nc, Vp, Pp, W.at(j, j + jb), batch, st);
     }
+    return true;
   };
-  factor_block(0, ms);
+  if (!factor_block(0, ms)) return false;
   for (int J = 0; J < n; J += QB) {
     const int jbB = std::min(QB, n - J);
     const int nc = n - J - jbB;
@@ -520,6 +530,7 @@ void geqrf(Context& c, int mtot, int n, int m_top, Mat W, double* tau, double* T
       factor_block(J + jbB, ms);
     }
   }
+  return true;
 }
 
 // Q = H_1 ... H_k applied to the identity, one 128-column block reflector at a time from the

@@ -3,6 +3,7 @@
 // a constant stride, runs on ctx.stream() and throws CudaFailure on error.
 #pragma once
 #include <cstdint>
+#include <functional>
 
 #include "context.h"
 
@@ -65,7 +66,10 @@ void trtri_lower(Context& c, int n, Mat L, Mat Y, int batch);
 // tau: n per batch entry; T: ceil(n/32) * 32 * 32 per batch entry.
 // The next panel is factored on a high-priority side stream while the rest of
 // the trailing matrix is updated (look-ahead of depth 1).
-void geqrf(Context& c, int mtot, int n, int m_top, Mat W, double* tau, double* T, int batch, bool top_tri = false);
+// keep_on: asked once the first of several panels is queued; false leaves the rest undone, and geqrf
+// returns false.
+bool geqrf(Context& c, int mtot, int n, int m_top, Mat W, double* tau, double* T, int batch, bool top_tri = false,
+           const std::function<bool()>& keep_on = nullptr);
 // Explicit Q (mtot x nq, nq >= n; default nq = n) from the n reflectors of geqrf
 // (mpdorgqr.f / dorgqr with N >= K).
 void orgqr(Context& c, int mtot, int n, int m_top, Mat W, const double* T, Mat Q, int batch, int nq = -1,

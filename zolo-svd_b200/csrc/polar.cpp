@@ -319,6 +319,19 @@ double norm2_upper(Context& c, int n, const double* W, int64_t ldw) {
   if (!(f > 0.0) || !std::isfinite(f)) return 1.0;
   return std::min(1.0, std::pow(f, 1.0 / 16.0) * (1.0 + 1e-4));
 }
+
+// The value that the GPU writes to *word, below zero until then (or the word as it stands once the
+// stream has nothing left to do).
+double known_norm(Context& c, const volatile double* word) {
+  for (unsigned spin = 1;; ++spin) {
+    const double v = *word;
+    if (!(v < 0.0)) return v;
+    if (spin % 256 == 0) {
+      if (cudaStreamQuery(c.stream()) != cudaErrorNotReady) return *word;
+      std::this_thread::yield();
+    }
+  }
+}
 }  // namespace
 
 int bounds(Context& c, int m, int n, double sigma, const double* dA, int64_t lda, BoundsMode mode, double* alpha,
@@ -330,9 +343,12 @@ int bounds(Context& c, int m, int n, double sigma, const double* dA, int64_t lda
   ck(scale_copy(m, n, 1.0, dA, lda, 0, X, ldx, 0, 1, -sigma, c.stream()));
   ck(frob2(m, n, X, ldx, part, scal, c.stream()));
   c.stats.launches += 3;
-  // scaled by 1 / ||A||_F on the device: the norms come back together at the end (each read-back
-  // left the GPU idle for 30 us); a zero or non-finite norm is found there
-  ck(scale_by_norm(m, n, scal, X, ldx, c.stream()));
+  // scaled by 1 / ||A||_F on the device, the norms read back together at the end (each read-back
+  // left the GPU idle for 30 us).  A zero or non-finite norm, after which the QR would be for nothing, is
+  // seen once the first panel is queued: the GPU has that to do meanwhile.
+  volatile double* early = c.norm_word();
+  *early = -1.0;
+  ck(scale_by_norm(m, n, scal, X, ldx, early, c.stream()));
   c.stats.launches++;
   if (mode == BOUNDS_PQDWHFACS) {
     double* colsum = c.buf("bnd_colsum", n);
@@ -343,7 +359,17 @@ int bounds(Context& c, int m, int n, double sigma, const double* dA, int64_t lda
   // inverse and R^{-1} as its transpose for ||R^{-1}||_1 and ||R^{-1}||_F
   double* tau = c.buf("bnd_tau", n);
   double* T = c.buf("bnd_t", static_cast<size_t>(npanels(n)) * 1024);
-  geqrf(c, m, n, -1, Mat{X, ldx, 0}, tau, T, 1);
+  auto usable = [&]() {
+    const double f = known_norm(c, early);
+    return f > 0.0 && std::isfinite(f);
+  };
+  if (!geqrf(c, m, n, -1, Mat{X, ldx, 0}, tau, T, 1, false, usable)) {
+    ck(cudaStreamSynchronize(c.stream()));
+    *alpha = std::sqrt(*early);
+    if (alpha_fro) *alpha_fro = *alpha;
+    *beta = 0.0;
+    return 1;
+  }
   double* Lt = c.buf("bnd_lt", static_cast<size_t>(ldn) * n);
   double* I = c.buf("bnd_i", static_cast<size_t>(ldn) * n);
   double* Ri = c.buf("bnd_rinv", static_cast<size_t>(ldn) * n);
