@@ -402,8 +402,10 @@ static void apply_panel(Context& c, const PanelRows& R, int jb, int ncols, Mat V
 // in 128-column blocks: while the trailing update fits beside the next panel the blocks' T factors
 // and products only lengthen the chain.  Measured, panelwise against blocks: QR of 1024 x 1024
 // 1.52 / 1.67 ms, 2048 x 2048 3.71 / 4.04, 4096 x 2048 7.6 / 5.7; forming Q, where nothing hides the
-// update, 512 x 512 0.147 / 0.157, 1024 x 1024 0.42 / 0.38, 2048 x 1024 0.86 / 0.55.  A batch of
-// 64 matrices of n <= 160 takes 1.73 ms with its buckets up to 1.5e6 panelwise, 1.77 with 5e5.
+// update, 512 x 512 0.147 / 0.157, 1024 x 1024 0.42 / 0.38, 2048 x 1024 0.86 / 0.55.  Batches of equal members form Q
+// panel by panel up to 1.5e6 entries of their stacks: whole batched solves with 6e5 to 1.4e6 entries
+// took 1 to 6 % less than in blocks for members of 64^2 to 160^2 and 300 x 100 (72 of 100^2 1.77 / 1.85 ms, 28 of
+// 160^2 1.87 / 1.93) and the same within 1 % for 250^2, 400^2 and 600 x 150, which lose up to 2 % at 4e6.
 static bool panelwise(int mtot, int n, int batch, bool qr) {
   const double one = static_cast<double>(mtot) * n, all = one * batch;
   return reflect_applies(mtot) && (qr ? all <= 4.5e6 : one <= 5e5 && all <= 1.5e6);
