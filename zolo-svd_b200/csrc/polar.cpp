@@ -76,6 +76,8 @@ constexpr int kNsMaxSteps = 12;
 // the iterate.  Costs in units of n^3 flops at the measured GEMM rate, from the kernel times
 // at n = 8192; the parts that scale with m are multiplied by m/n.
 constexpr double kConChol = 12.0;
+// Two-factor form: up to this CON by products with L^-T and L^-1, above it by substitution (spd_solve).
+constexpr double kConInverse = 12.0;
 class TermPlanner {
  public:
   // `mixed`: the Cholesky iterations and Newton-Schulz steps run their products on the
@@ -259,10 +261,13 @@ void newton_schulz_finish(Context& c, int m, int n, double* X, int64_t ldx, Mat 
 }
 
 // Z(b) = X W_b^{-1} (left = false) or W_b^{-1} X (left = true, square X), from Y_b = L_b^{-1} of
-// W_b = L_b L_b^T: two products with a triangular factor.  W_b is the shifted Gram matrix of a
-// Cholesky-form step, whose L_b is well conditioned (QDWH: c <= 100, so at most 10), and a
-// triangular inverse applied to X is then as accurate as a substitution.  The substitution by
-// recursion was a chain of 62 narrow products at n = 1024; with Y_b from the factorization's own
+// W_b = L_b L_b^T: two products with a triangular factor.  For the well-conditioned L_b of QDWH (c <= 100: at most
+// 10) and of Zolo-PD up to CON = kConInverse, where a triangular inverse applied to X is as accurate as a
+// substitution.  Above it is not, most of all with the mixed form's products, which are accurate normwise only:
+// against substitution the default form's backward error grew from 3.5e-15 to 1.1e-14 in FP64 (700 x 600, r = 3,
+// CON = 343) and from 3.0e-15 to 5.0e-14 mixed (2400 x 2304, r = 8, CON = 236), and to 5.6e-15 at CON = 76;
+// over 525 solves with products up to CON = 12 it is that of substitution.
+// The substitution by recursion is a chain of 62 narrow products at n = 1024; with Y_b from the factorization's own
 // recursion QDWH n = 1024 went from 11.9 to 10.7 ms, a batch of 512 from 262 to 256.
 // strideX: X of batch entry b at X + b*strideX (0: one X shared by the r terms).
 void spd_solve(Context& c, int m, int n, const double* X, int64_t ldx, Mat Y, Mat Z, int batch, bool left,
@@ -277,6 +282,29 @@ void spd_solve(Context& c, int m, int n, const double* X, int64_t ldx, Mat Y, Ma
     gemm(c, 0, 0, n, m, n, 1.0, Y, Xb, 0.0, P, batch, nullptr, 0, 0, nullptr, 1);
     gemm(c, 1, 0, n, m, n, 1.0, Y, P, 0.0, Z, batch, nullptr, 0, 2);
   }
+}
+
+
+// The same by substitution with L_b (X shared by the batch), for factors that are not that well conditioned.
+void spd_substitute(Context& c, int m, int n, const double* X, int64_t ldx, Mat Lw, DiagInv D, Mat Z, int batch,
+                    bool left) {
+  const int64_t ldm = even(m);
+  Mat Xc{c.buf("Xc", static_cast<size_t>(ldm) * n * batch), ldm, ldm * n};
+  Mat Y{c.buf("Y", static_cast<size_t>(ldm) * n * batch), ldm, ldm * n};
+  if (!left) {
+    ck(scale_copy(m, n, 1.0, X, ldx, 0, Xc.p, Xc.ld, Xc.stride, batch, 0.0, c.stream()));
+    c.stats.launches++;
+    trsm_rlt(c, m, n, Lw, Xc, Y, batch, D);
+    trsm_rln(c, m, n, Lw, Y, Z, batch, D);
+    return;
+  }
+  // W^{-1} X = (X^T W^{-1})^T, X square: transposed in, solved from the right, transposed out
+  for (int b = 0; b < batch; ++b) ck(transpose(m, n, X, ldx, Xc.p + b * Xc.stride, Xc.ld, c.stream()));
+  trsm_rlt(c, n, m, Lw, Xc, Y, batch, D);
+  trsm_rln(c, n, m, Lw, Y, Xc, batch, D);
+  for (int b = 0; b < batch; ++b)
+    ck(transpose(n, m, Xc.p + b * Xc.stride, Xc.ld, Z.p + b * Z.stride, Z.ld, c.stream()));
+  c.stats.launches += 2 * batch;
 }
 
 }  // namespace
@@ -684,8 +712,16 @@ int zolo_pd(Context& c, char sym, int rk, int m, int n, double alpha, double bet
       ck(shift_lower(n, G.p, G.ld, Wc.p, Wc.ld, Wc.stride, dvec, rk_it, c.stream()));
       ck(cudaMemsetAsync(dinfo, 0, sizeof(int) * rk_it, c.stream()));
       c.stats.launches += 2;
-      Mat Y{c.buf("zc_y", static_cast<size_t>(ldn) * n * rk_it), ldn, ldn * n};
-      potrf_inv(c, n, Wc, Y, rk_it, dinfo);
+      const bool by_inverse = inverse_form || con <= kConInverse;
+      Mat Y{nullptr, ldn, ldn * n};
+      DiagInv Dz{nullptr, static_cast<int64_t>(nblocks(n)) * 4096};
+      if (by_inverse) {
+        Y.p = c.buf("zc_y", static_cast<size_t>(ldn) * n * rk_it);
+        potrf_inv(c, n, Wc, Y, rk_it, dinfo);
+      } else {
+        Dz.p = c.buf("dinv", static_cast<size_t>(Dz.stride) * rk_it);
+        potrf(c, n, Wc, rk_it, dinfo, Dz);
+      }
       const int pinfo = injected_info(c, it, read_info(c, dinfo, rk_it));
       if (pinfo != 0) {
         if (c.stats.info == 0) c.stats.info = pinfo;
@@ -710,13 +746,14 @@ int zolo_pd(Context& c, char sym, int rk, int m, int n, double alpha, double bet
         c.stats.flops += canonical;
         c.stats.flops_exec_delta += 3.0 * dmx * dn * dn + rk_it * dn * dn * dn - canonical;
       } else {
-        spd_solve(c, mx, n, X, ldx, Y, Z, rk_it, left);
+        if (by_inverse) spd_solve(c, mx, n, X, ldx, Y, Z, rk_it, left);
+        else spd_substitute(c, mx, n, X, ldx, Wc, Dz, Z, rk_it, left);
         for (int b = 0; b < rk_it; ++b) hv[16 + b] = -coeff[2 * rk_it + b];
         c.stats.chol_iterations++;
         if (it < 16) c.stats.branch[it] = 2;
         c.stats.flops += static_cast<double>(m) * n * n +
                          rk_it * (static_cast<double>(n) * n * n / 3.0 + 2.0 * m * static_cast<double>(n) * n);
-        c.stats.flops_exec_delta += rk_it * static_cast<double>(n) * n * n / 3.0;  // the factors' inverses
+        if (by_inverse) c.stats.flops_exec_delta += rk_it * static_cast<double>(n) * n * n / 3.0;  // the factors' inverses
       }
     }
     const double fone = zolo_fone(coeff.data(), rk_it);
