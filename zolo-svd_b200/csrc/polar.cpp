@@ -289,8 +289,9 @@ void spd_solve(Context& c, int m, int n, const double* X, int64_t ldx, Mat Y, Ma
 void spd_substitute(Context& c, int m, int n, const double* X, int64_t ldx, Mat Lw, DiagInv D, Mat Z, int batch,
                     bool left) {
   const int64_t ldm = even(m);
-  Mat Xc{c.buf("Xc", static_cast<size_t>(ldm) * n * batch), ldm, ldm * n};
-  Mat Y{c.buf("Y", static_cast<size_t>(ldm) * n * batch), ldm, ldm * n};
+  // the buffers of the other route: a solve that takes both holds two per term
+  Mat Xc{c.buf("spd_p", static_cast<size_t>(ldm) * n * batch), ldm, ldm * n};
+  Mat Y{c.buf("zc_y", static_cast<size_t>(ldm) * n * batch), ldm, ldm * n};
   if (!left) {
     ck(scale_copy(m, n, 1.0, X, ldx, 0, Xc.p, Xc.ld, Xc.stride, batch, 0.0, c.stream()));
     c.stats.launches++;
