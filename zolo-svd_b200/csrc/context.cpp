@@ -195,7 +195,7 @@ Profiler::~Profiler() {
   for (auto e : pool) cudaEventDestroy(e);
 }
 
-double* Context::dscal() { return buf("__scal", 64); }
+double* Context::dscal() { return buf("__scal", 192); }
 double* Context::dpartial() { return buf("__partial", 4096); }
 int* Context::dinfo() { return ibuf("__info", 1024); }
 

@@ -164,7 +164,7 @@ class Context {
   void drop_graphs();
 
   // small device scalars / partial sums
-  double* dscal();     // 64 doubles
+  double* dscal();     // 192 doubles
   double* dpartial();  // 4096 doubles
   int* dinfo();        // 1024 ints
   int* oz_status_word();  // status of the INT8-emulated products (zeroed when allocated)

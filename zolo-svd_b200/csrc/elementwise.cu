@@ -138,16 +138,19 @@ __global__ void max_kernel(const double* v, int count, double* out) {
   if (threadIdx.x == 0) out[0] = sh[0];
 }
 
-// X_new = cx*X + cz*sum_q Z_q ; partial = ||X_new - X||^2 per block.  In place on X.
+// X_new = cx*X + cz*sum_q Z_q ; partial = ||X_new - X||^2 per block.  In place on X.  X stays as it is when one
+// of info[0 .. ninfo) is not zero (a select, not a branch: the loads are in flight together).
 __global__ void combine_kernel(int m, int n, double* X, int64_t ldx, const double* Z,
                                int64_t ldz, int64_t strideZ, int nz, double cx, double cz,
-                               const double* cz_vec, double* partial) {
+                               const double* cz_vec, double* partial, const int* info, int ninfo) {
   dependency_wait();
   release_dependents();
   __shared__ double sh[TPB / 32];
   double s = 0.0;
+  int stop = 0;
+  for (int k = 0; k < ninfo; ++k) stop |= info[k];
   auto update = [&](int i, int j, double x, double z) {
-    const double xn = cx * x + (cz_vec ? z : z * cz);
+    const double xn = stop ? x : cx * x + (cz_vec ? z : z * cz);
     const double d = x - xn;
     s += d * d;
     X[i + j * ldx] = xn;
@@ -361,9 +364,9 @@ cudaError_t norm1(int m, int n, const double* X, int64_t ldx, double* colsum, do
 
 cudaError_t combine_update(int m, int n, double* X, int64_t ldx, const double* Z, int64_t ldz, int64_t strideZ,
                            int nz, double cx, double cz, const double* cz_vec, double* partial, double* err2,
-                           cudaStream_t st) {
+                           cudaStream_t st, const int* info, int ninfo) {
   const int blocks = std::min(grid_for(static_cast<int64_t>(m) * n), 1024);
-  cudaError_t e = launch_dependent(combine_kernel, dim3(blocks), dim3(TPB), 0, st, dim3(1), m, n, X, ldx, Z, ldz, strideZ, nz, cx, cz, cz_vec, partial);
+  cudaError_t e = launch_dependent(combine_kernel, dim3(blocks), dim3(TPB), 0, st, dim3(1), m, n, X, ldx, Z, ldz, strideZ, nz, cx, cz, cz_vec, partial, info, ninfo);
   if (e != cudaSuccess) return e;
   return reduce_sum(partial, blocks, err2, st);
 }

@@ -86,10 +86,12 @@ cudaError_t frob2(int m, int n, const double* X, int64_t ldx, double* partial, d
 cudaError_t norm1(int m, int n, const double* X, int64_t ldx, double* colsum, double* out,
                   cudaStream_t st);
 // X <- cx X + sum_q w_q Z_q, w_q = cz_vec[q] (device) or cz; err2 = ||X_new - X_old||_F^2
-// (FormX2 of Zolo-PD with w_q = a_q / FONE, cx = 1/FONE; QDWH update with cx = bkk, cz = akk)
+// (FormX2 of Zolo-PD with w_q = a_q / FONE, cx = 1/FONE; QDWH update with cx = bkk, cz = akk).  X stays as it
+// is when one of the ninfo words at info (device) is not zero.
 cudaError_t combine_update(int m, int n, double* X, int64_t ldx, const double* Z, int64_t ldz,
                            int64_t strideZ, int nz, double cx, double cz, const double* cz_vec,
-                           double* partial, double* err2, cudaStream_t st);
+                           double* partial, double* err2, cudaStream_t st, const int* info = nullptr,
+                           int ninfo = 0);
 // H = (B + B^T)/2 (in place on an n x n matrix).
 cudaError_t symmetrize(int n, double* B, int64_t ldb, cudaStream_t st);
 // B = scale * triu(A) (n x n; zero below the diagonal)

@@ -486,107 +486,108 @@ int qdwh(Context& c, int m, int n, const double* dA, int64_t lda, double* dQ, in
 
   // The loop ends on ||X_{k+1} - X_k||_F only once L has converged, and L follows from L_0 alone: up
   // to there no step waits for the host.  Errors and Cholesky INFO stay on the device, a slot a
-  // step, and come back together; a failed factorization is found then and the loop runs again
-  // from X_0, reading INFO before each solve.  (One read-back and one wait a step left the GPU idle
+  // step, and come back together.  After a failed factorization no step changes X any more (the update
+  // reads the INFOs), so that X is still the failed step's when the host sees it, and the loop goes on
+  // there with the QR form.  (One read-back and one wait a step left the GPU idle
   // for 35 us each: QDWH n = 96 0.98 -> 0.77 ms.)
-  constexpr int kSlots = 16;
+  constexpr int kMaxSteps = 100;  // as many slots: dscal has 192
   double* errs = scal + 32;
-  const Stats stats0 = c.stats;
-  const int t_loop = marks.mark(c.stream());
-  int it = 0, t_end = t_loop;
-  double err = 1.0;
-  auto iterate = [&](bool careful) -> bool {
-    std::vector<int> t_step{marks.mark(c.stream())};
-    ck(scale_copy(m, n, 1.0, Ain, ldx, 0, X, ldx, 0, 1, -o.sigma, c.stream()));
-    ck(scale_copy(m, n, 1.0 / alpha, X, ldx, 0, X, ldx, 0, 1, 0.0, c.stream()));
-    ck(cudaMemsetAsync(dinfo, 0, sizeof(int) * kSlots, c.stream()));
-    c.stats.launches += 3;
-    double herr[kSlots];
-    int hinfo[kSlots], have = 0;  // steps read back
-    // errors and INFO of the steps so far; false when a factorization failed
-    auto read_back = [&]() {
-      ck(cudaMemcpyAsync(herr, errs, sizeof(herr), cudaMemcpyDeviceToHost, c.stream()));
-      ck(cudaMemcpyAsync(hinfo, dinfo, sizeof(hinfo), cudaMemcpyDeviceToHost, c.stream()));
-      ck(cudaStreamSynchronize(c.stream()));
-      have = it;
-      for (int k = 0; k < std::min(it, kSlots); ++k) {
-        if (!careful && c.stats.branch[k] == 2 && injected_info(c, k, hinfo[k]) != 0) return false;
-        c.stats.err[k] = std::sqrt(herr[k]);
-      }
-      return true;
-    };
-    double lowk = beta, err2 = std::fabs(1.0 - lowk);
-    it = 0;
-    err = 1.0;
-    while ((o.maxit < 0 || it <= o.maxit) && it < 100) {
-      const int slot = std::min(it, kSlots - 1);
-      if (it > 0 && (careful || err2 <= tol1)) {
-        if (!careful && !read_back()) return false;
-        err = careful ? std::sqrt(d2h(c, errs + std::min(it - 1, kSlots - 1))) : c.stats.err[it - 1];
-        if (!(err > tol2 || err2 > tol1)) break;
-      }
-      if (!careful && it == kSlots) return false;  // no slot for another step
-      double ak, bk, ckk, lnext;
-      qdwh_weights(lowk, &ak, &bk, &ckk, &lnext);
-      lowk = lnext;
-      double akk, bkk;
-      bool use_qr = ckk > 100.0;
-      if (!use_qr) {
-        OzScope mixed_ch(c, c.zolo_mixed >= 1);  // the mixed form's products of this Cholesky step
-        gemm(c, 1, 0, n, n, m, ckk, Mat{X, ldx, 0}, Mat{X, ldx, 0}, 0.0, G, 1, nullptr, 1, 0);
-        ck(add_diag(n, G.p, G.ld, 1.0, c.stream()));
-        c.stats.launches++;
-        if (careful) {
-          ck(cudaMemsetAsync(dinfo + slot, 0, sizeof(int), c.stream()));
-          c.stats.launches++;
-        }
-        potrf_inv(c, n, G, Y, 1, dinfo + slot);
-        const int pinfo = careful ? injected_info(c, it, read_info(c, dinfo + slot, 1)) : 0;
-        if (pinfo != 0) {
-          // not numerically SPD: redo this step with the QR form (the reference ignores PDPOSV's INFO)
-          if (c.stats.info == 0) c.stats.info = pinfo;
-          use_qr = true;
-        } else {
-          spd_solve(c, m, n, X, ldx, Y, Z, 1, left);
-          akk = ak - bk / ckk;
-          bkk = bk / ckk;
-          c.stats.chol_iterations++;
-          if (it < 16) c.stats.branch[it] = 2;
-          c.stats.flops += 2.0 * m * static_cast<double>(n) * n + static_cast<double>(n) * n * n / 3.0 +
-                           static_cast<double>(m) * n * n;
-          c.stats.flops_exec_delta += static_cast<double>(n) * n * n / 3.0;  // the factor's inverse
-        }
-      }
-      if (use_qr) {
-        const double sck = std::sqrt(ckk);
-        ck(form_stack(m, mp, n, X, ldx, W.p, W.ld, 0, nullptr, 1.0 / sck, 1, c.stream()));
-        c.stats.launches++;
-        geqrf(c, mp + n, n, mp, W, tau, T, 1);
-        orgqr(c, mp + n, n, mp, W, T, Qf, 1);
-        q1q2t(c, m, mp, n, Qf, Z, 1);
-        akk = (ak - bk / ckk) / sck;
-        bkk = bk / ckk;
-        c.stats.qr_iterations++;
-        if (it < 16) c.stats.branch[it] = 1;
-        c.stats.flops += 4.0 * m * static_cast<double>(n) * n + static_cast<double>(n) * n * n;
-      }
-      ck(combine_update(m, n, X, ldx, Z.p, Z.ld, 0, 1, bkk, akk, nullptr, part, errs + slot, c.stream()));
-      c.stats.launches += 2;
-      if (it < 16) c.stats.con[it] = ckk;
-      t_step.push_back(marks.mark(c.stream()));
-      ++it;
-      err2 = std::fabs(1.0 - lowk);
-    }
-    if (have != it && !read_back()) return false;
-    if (it > 0) err = std::sqrt(herr[std::min(it, kSlots) - 1]);
-    t_end = t_step.back();
-    for (int k = 0; k < std::min(it, 16); ++k) c.stats.ms_step[k] = marks.ms(t_step[k], t_step[k + 1]);
-    return true;
+  struct Before {  // what a step starts from
+    Stats stats;
+    double lowk;
+    bool chol;
   };
-  if (!iterate(false)) {
-    c.stats = stats0;
-    iterate(true);
+  std::vector<Before> before;
+  const int t_loop = marks.mark(c.stream());
+  std::vector<int> t_step{t_loop};
+  ck(scale_copy(m, n, 1.0, Ain, ldx, 0, X, ldx, 0, 1, -o.sigma, c.stream()));
+  ck(scale_copy(m, n, 1.0 / alpha, X, ldx, 0, X, ldx, 0, 1, 0.0, c.stream()));
+  ck(cudaMemsetAsync(dinfo, 0, sizeof(int) * kMaxSteps, c.stream()));
+  c.stats.launches += 3;
+  double herr[kMaxSteps];
+  int hinfo[kMaxSteps];
+  // errors and INFO of the steps so far; the first step whose factorization failed, or -1
+  auto read_back = [&](int steps) {
+    ck(cudaMemcpyAsync(herr, errs, sizeof(double) * steps, cudaMemcpyDeviceToHost, c.stream()));
+    ck(cudaMemcpyAsync(hinfo, dinfo, sizeof(int) * steps, cudaMemcpyDeviceToHost, c.stream()));
+    ck(cudaStreamSynchronize(c.stream()));
+    for (int k = 0; k < steps; ++k) {
+      if (before[k].chol && hinfo[k] != 0) return k;
+      if (k < 16) c.stats.err[k] = std::sqrt(herr[k]);
+    }
+    return -1;
+  };
+  double lowk = beta, err = 1.0;
+  int it = 0, failed = -1, first_chol = kMaxSteps;
+  while (true) {
+    const bool over = (o.maxit >= 0 && it > o.maxit) || it >= kMaxSteps;
+    const bool converged = std::fabs(1.0 - lowk) <= tol1;
+    if (it > 0 && (over || converged)) {
+      const int k = read_back(it);
+      if (k >= 0) {
+        // not numerically SPD: this step again with the QR form (the reference ignores PDPOSV's INFO)
+        const int64_t launches = c.stats.launches;
+        c.stats = before[k].stats;
+        c.stats.launches = launches;
+        if (c.stats.info == 0) c.stats.info = hinfo[k];
+        lowk = before[k].lowk;
+        before.resize(k);
+        t_step.resize(k + 1);
+        it = failed = k;
+        ck(cudaMemsetAsync(dinfo + k, 0, sizeof(int) * (kMaxSteps - k), c.stream()));
+        c.stats.launches++;
+        continue;
+      }
+      err = std::sqrt(herr[it - 1]);
+      if (converged && !(err > tol2)) break;
+    }
+    if (over) break;
+    before.push_back(Before{c.stats, lowk, false});
+    double ak, bk, ckk, lnext;
+    qdwh_weights(lowk, &ak, &bk, &ckk, &lnext);
+    lowk = lnext;
+    double akk, bkk;
+    if (ckk <= 100.0 && it != failed) {
+      before[it].chol = true;
+      first_chol = std::min(first_chol, it);
+      OzScope mixed_ch(c, c.zolo_mixed >= 1);  // the mixed form's products of this Cholesky step
+      gemm(c, 1, 0, n, n, m, ckk, Mat{X, ldx, 0}, Mat{X, ldx, 0}, 0.0, G, 1, nullptr, 1, 0);
+      ck(add_diag(n, G.p, G.ld, 1.0, c.stream()));
+      c.stats.launches++;
+      if (const int bad = injected_info(c, it, 0))
+        ck(cudaMemcpyAsync(dinfo + it, &bad, sizeof(int), cudaMemcpyHostToDevice, c.stream()));
+      potrf_inv(c, n, G, Y, 1, dinfo + it);
+      spd_solve(c, m, n, X, ldx, Y, Z, 1, left);
+      akk = ak - bk / ckk;
+      bkk = bk / ckk;
+      c.stats.chol_iterations++;
+      if (it < 16) c.stats.branch[it] = 2;
+      c.stats.flops += 2.0 * m * static_cast<double>(n) * n + static_cast<double>(n) * n * n / 3.0 +
+                       static_cast<double>(m) * n * n;
+      c.stats.flops_exec_delta += static_cast<double>(n) * n * n / 3.0;  // the factor's inverse
+    } else {
+      const double sck = std::sqrt(ckk);
+      ck(form_stack(m, mp, n, X, ldx, W.p, W.ld, 0, nullptr, 1.0 / sck, 1, c.stream()));
+      c.stats.launches++;
+      geqrf(c, mp + n, n, mp, W, tau, T, 1);
+      orgqr(c, mp + n, n, mp, W, T, Qf, 1);
+      q1q2t(c, m, mp, n, Qf, Z, 1);
+      akk = (ak - bk / ckk) / sck;
+      bkk = bk / ckk;
+      c.stats.qr_iterations++;
+      if (it < 16) c.stats.branch[it] = 1;
+      c.stats.flops += 4.0 * m * static_cast<double>(n) * n + static_cast<double>(n) * n * n;
+    }
+    const int from = std::min(first_chol, it + 1);
+    ck(combine_update(m, n, X, ldx, Z.p, Z.ld, 0, 1, bkk, akk, nullptr, part, errs + it, c.stream(), dinfo + from,
+                      it + 1 - from));
+    c.stats.launches += 2;
+    if (it < 16) c.stats.con[it] = ckk;
+    t_step.push_back(marks.mark(c.stream()));
+    ++it;
   }
+  const int t_end = t_step.back();
+  for (int k = 0; k < std::min(it, 16); ++k) c.stats.ms_step[k] = marks.ms(t_step[k], t_step[k + 1]);
   c.stats.ms_iter = marks.ms(t_loop, t_end);
   c.stats.iterations = it;
   c.stats.last_err = err;
