@@ -56,11 +56,16 @@ using CfgTiny = Cfg<32, 32, 2, 2, 4, 4>;       // products too small to fill the
 struct KParams {
   GemmArgs g;
   int tiles_m, tiles_n;
-  int splitk;
+  int splitk;   // slices of K, blockIdx.y
+  int cluster;  // the slices that one cluster sums: all of them, or groups whose sums go to P
+  double* P;    // partial sums of the groups: M x N (ld ldp) for each group and batch entry
+  int64_t ldp;
   int stage_c;  // C copied to shared memory beside the first K tiles (rank-k updates)
 };
 
-template <class C, bool TA, bool TB, bool V16>
+// GROUPS: a kernel of its own, so that the general one's code stays as it is (with both in one, 128 x 1024 x 4096
+// went from 61.5 to 69.5 us)
+template <class C, bool TA, bool TB, bool V16, bool GROUPS>
 __global__ void __launch_bounds__(C::NT, C::MINB) dgemm_kernel(KParams kp) {
   constexpr int NT = C::NT;
   constexpr int BM = C::BM, BN = C::BN, MI = C::MI, NJ = C::NJ;
@@ -247,9 +252,10 @@ __global__ void __launch_bounds__(C::NT, C::MINB) dgemm_kernel(KParams kp) {
 
   // ---- epilogue ----
   if (kp.splitk > 1) {
-    // the slices of a tile are one cluster: every CTA leaves its partial tile in shared memory,
+    // the slices of a tile are one cluster, or a few: every CTA leaves its partial tile in shared memory,
     // and each then sums its share of the columns over the cluster in slice order and writes it
-    // (a pass through global scratch cost a second launch, 2.5 us and its gap)
+    // (a pass through global scratch costs a second launch, 2.5 us and its gap, so only where one
+    // cluster leaves most SMs idle: splitk_reduce_kernel)
     constexpr int LDP = BM + 2;
     static_assert(BN * LDP * 8 <= C::smem(TA, TB), "partial tile fits the pipeline's buffers");
     cg::cluster_group cluster = cg::this_cluster();
@@ -265,10 +271,13 @@ __global__ void __launch_bounds__(C::NT, C::MINB) dgemm_kernel(KParams kp) {
           *reinterpret_cast<double2*>(P + r + (c + h) * LDP) = make_double2(acc[i][j][h], acc[i][j][2 + h]);
       }
     cluster.sync();
-    const double al = p.alpha * (p.alpha_vec ? p.alpha_vec[bz] : 1.0);
-    double* Cb = p.C + static_cast<int64_t>(bz) * p.strideC;
-    const int S = kp.splitk, per = (BN + S - 1) / S;
-    const int c0 = split * per, c1 = min(BN, c0 + per);
+    const double al = GROUPS ? 1.0 : p.alpha * (p.alpha_vec ? p.alpha_vec[bz] : 1.0);
+    const double be = GROUPS ? 0.0 : p.beta;
+    const int64_t ldc = GROUPS ? kp.ldp : p.ldc;
+    double* Cb = GROUPS ? kp.P + (static_cast<int64_t>(split / kp.cluster) * p.batch + bz) * kp.ldp * N
+                        : p.C + static_cast<int64_t>(bz) * p.strideC;
+    const int S = GROUPS ? kp.cluster : kp.splitk, per = (BN + S - 1) / S;
+    const int c0 = (GROUPS ? split % S : split) * per, c1 = min(BN, c0 + per);
     for (int e = tid; e < (c1 - c0) * (BM / 2); e += NT) {
       const int r = (e % (BM / 2)) * 2, c = c0 + e / (BM / 2);
       double s0 = 0.0, s1 = 0.0;
@@ -280,9 +289,9 @@ __global__ void __launch_bounds__(C::NT, C::MINB) dgemm_kernel(KParams kp) {
       }
       const int gr = m0 + r, gc = n0 + c;
       if (gc >= N) continue;
-      double* dst = Cb + gr + static_cast<int64_t>(gc) * p.ldc;
-      if (gr < M && (!p.tri || gr >= gc)) dst[0] = p.beta != 0.0 ? fma(p.beta, dst[0], al * s0) : al * s0;
-      if (gr + 1 < M && (!p.tri || gr + 1 >= gc)) dst[1] = p.beta != 0.0 ? fma(p.beta, dst[1], al * s1) : al * s1;
+      double* dst = Cb + gr + static_cast<int64_t>(gc) * ldc;
+      if (gr < M && (!p.tri || gr >= gc)) dst[0] = be != 0.0 ? fma(be, dst[0], al * s0) : al * s0;
+      if (gr + 1 < M && (!p.tri || gr + 1 >= gc)) dst[1] = be != 0.0 ? fma(be, dst[1], al * s1) : al * s1;
     }
     cluster.sync();  // no CTA leaves while others read its partial tile
     return;
@@ -324,17 +333,42 @@ __global__ void __launch_bounds__(C::NT, C::MINB) dgemm_kernel(KParams kp) {
     }
 }
 
-template <class C, bool TA, bool TB, bool V16>
-cudaError_t launch_t(const KParams& kp, dim3 grid, cudaStream_t st) {
+// C = beta C + alpha times the sum of the groups' partial sums, in their order
+__global__ void splitk_reduce_kernel(GemmArgs p, int groups, const double* P, int64_t ldp) {
+  dependency_wait();
+  release_dependents();
+  const int bz = blockIdx.y;
+  const double alpha = p.alpha * (p.alpha_vec ? p.alpha_vec[bz] : 1.0);
+  const int64_t one = ldp * p.N, group = one * p.batch;
+  const double* Pb = P + bz * one;
+  double* C = p.C + bz * p.strideC;
+  for_entries(p.M, p.N, [&](int i, int j) {
+    if (p.tri && i < j) return;
+    const double* src = Pb + i + j * ldp;
+    double s = 0.0;
+#pragma unroll 4
+    for (int q = 0; q < groups; ++q) s += src[q * group];
+    double* dst = C + i + j * p.ldc;
+    *dst = p.beta != 0.0 ? fma(p.beta, *dst, alpha * s) : alpha * s;
+  });
+}
+
+template <class C, bool TA, bool TB, bool V16, bool GROUPS>
+cudaError_t launch_g(const KParams& kp, dim3 grid, cudaStream_t st) {
   static std::atomic<int> attr_set[kMaxDevices];
   const cudaError_t attr = once_per_device(attr_set, [] {
-    return cudaFuncSetAttribute(dgemm_kernel<C, TA, TB, V16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(dgemm_kernel<C, TA, TB, V16, GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 C::smem(TA, TB) + C::SMEM_C);
   });
   if (attr != cudaSuccess) return attr;
-  return launch_dependent(dgemm_kernel<C, TA, TB, V16>, grid, dim3(C::NT),
-                          C::smem(TA, TB) + (kp.stage_c ? C::SMEM_C : 0), st, dim3(1, kp.splitk, 1),
-                          kp);
+  return launch_dependent(dgemm_kernel<C, TA, TB, V16, GROUPS>, grid, dim3(C::NT),
+                          C::smem(TA, TB) + (kp.stage_c ? C::SMEM_C : 0), st, dim3(1, kp.cluster, 1), kp);
+}
+
+template <class C, bool TA, bool TB, bool V16>
+cudaError_t launch_t(const KParams& kp, dim3 grid, cudaStream_t st) {
+  return kp.cluster < kp.splitk ? launch_g<C, TA, TB, V16, true>(kp, grid, st)
+                                : launch_g<C, TA, TB, V16, false>(kp, grid, st);
 }
 
 template <class C, bool V16>
@@ -418,13 +452,12 @@ int split_general(int64_t ctas, int kt, int sms) {
   return best;
 }
 
-// Split K only when the tile grid cannot fill the GPU; pick the split (the CTAs of one portable
+// Split K in one cluster only when the tile grid cannot fill the GPU; pick the split (the CTAs of a portable
 // cluster, 8 at most) that fills whole waves (sms * resident CTAs per SM) best, with at least 8
 // K tiles per split (4 of the 32 x 32 tiles).
-int choose_splitk(const GemmArgs& a, int sms) {
+int choose_splitk(const GemmArgs& a, int cfg, int sms) {
   if (a.splitk >= 1) return a.splitk;
   int BM, BN, per_sm;
-  const int cfg = pick_cfg(a);
   tile_dims(cfg, &BM, &BN, &per_sm);
   const int tm = (a.M + BM - 1) / BM, tn = (a.N + BN - 1) / BN;
   const int64_t tiles = a.tri ? static_cast<int64_t>(tm) * (tm + 1) / 2 : static_cast<int64_t>(tm) * tn;
@@ -451,7 +484,74 @@ int choose_splitk(const GemmArgs& a, int sms) {
   return best;
 }
 
+bool long_k(const GemmArgs& a) { return a.K > 127 * BK && a.splitk < 1 && !a.kfrom_n && !a.kto_m; }
+
+struct Plan {
+  int cfg, cluster, groups;  // tile shape, slices of K summed inside a cluster, clusters a tile
+};
+
+// A long K over few tiles: one cluster of 8 CTAs a tile leaves most SMs idle, and clusters of 8 do not fill the SMs
+// evenly.  From K = 2048 (kt = 128) on and up to two tiles an SM, groups of clusters share a tile, their sums
+// going through scratch in global memory: a second launch of 2 to 5 us, so only where it saves more.
+// About 512 CTAs, of at least 4 K tiles (8 of the larger tiles); more for a longer K, and not a second wave of a
+// few (64 x 64 tiles are resident four to an SM); clusters of 2 from 16 tiles or so on.  32 x 32 tiles serve the
+// smallest outputs, 64 x 64 with four warps the rest; 32 x 64 only M <= 32 with N from 4096 on.
+// Measured in one cluster (the tiles and slices of choose_splitk) against this, the chain drained between, us:
+// 32 x 32 x 4096 20.6 / 10.4, 32 x 512 x 8192 41 / 23, 512 x 64 x 8192 66 / 35, 128 x 512 x 8192 105 / 56,
+// 64 x 64 x 65536 242 / 33, 128 x 2048 x 8192 184 / 170, 8192 x 64 x 8192 367 / 316, 1000 x 1000 x 8192 680 / 602,
+// lower triangle of 512 x 512 x 8192 144 / 103; at K = 1024 groups save nothing (32 x 32 10.3 / 10.3,
+// 128 x 1024 20.6 / 22.7).
+Plan plan_gemm(const GemmArgs& a, int sms) {
+  Plan now{pick_cfg(a), 1, 1};
+  now.cluster = choose_splitk(a, now.cfg, sms);
+  if (!long_k(a)) return now;
+  const int kt = (a.K + BK - 1) / BK;
+  auto tiles = [&](int bm, int bn) {
+    const int64_t tm = (a.M + bm - 1) / bm, tn = (a.N + bn - 1) / bn;
+    return (a.tri ? tm * (tm + 1) / 2 : tm * tn) * a.batch;
+  };
+  const int64_t t64 = tiles(64, 64);
+  int cfg = now.cfg;
+  if (a.M <= 32) cfg = a.N < 4096 ? 4 : 1;
+  else if (a.tri) cfg = t64 <= 10 || (t64 <= 36 && kt < 512) ? 4 : 0;
+  else if (kt < 512) cfg = t64 <= 16 ? 4 : (t64 >= 48 && cfg == 2 ? 0 : cfg);
+  else if (t64 >= 8) cfg = 0;
+  int bm, bn, per_sm;
+  tile_dims(cfg, &bm, &bn, &per_sm);
+  const int64_t n = tiles(bm, bn);
+  if (n > sms) {
+    // split_general's slices in clusters of 2, eight of them from 200 tiles on (1000 x 1000 x 20000 1461 / 1431 us)
+    const bool groups = cfg == 0 && now.cfg == 0 && !a.tri && kt >= 256 && n <= 2 * sms && now.cluster >= 4;
+    return groups ? Plan{0, 2, n >= 200 ? 4 : now.cluster / 2} : now;
+  }
+  const bool wide = n >= 96;
+  if (n >= 48) {
+    if (cfg == 4) return !wide ? Plan{4, 8, 1} : (a.tri || kt < 512 ? Plan{4, 4, 1} : Plan{4, 2, 4});
+    if (kt < (wide ? 256 : 512)) return cfg == 1 ? Plan{1, 4, 1} : (cfg != now.cfg ? Plan{cfg, 8, 1} : now);
+    if (wide) return a.tri ? now : Plan{cfg, 2, 4};
+    return n > 64 && cfg == 0 ? Plan{0, 4, 8} : Plan{cfg, 2, 8};
+  }
+  if (n > 16 && kt < (a.tri ? 256 : 512)) return cfg == 4 ? Plan{4, 8, 1} : now;
+  if (n > 24 && cfg != 4) return Plan{cfg, 2, n <= 32 ? 16 : 8};
+  const int min_kt = cfg == 4 ? 4 : 8;
+  const int64_t target = cfg == 4 || kt < 1024 ? 512 : (kt < 4096 ? 1024 : 2048);
+  int slices = 1;
+  auto more = [&] { return slices < 128 && kt / (2 * slices) >= min_kt; };
+  while (n * slices < target && more()) slices *= 2;
+  if (cfg != 4 && n * slices > 528 && n * slices <= 640 && more()) slices *= 2;
+  return slices <= 16 ? Plan{cfg, 2, slices / 2} : Plan{cfg, 8, slices / 8};
+}
+
+size_t scratch_elems(const GemmArgs& a, const Plan& p) {
+  return p.groups > 1 ? static_cast<size_t>(p.groups) * a.batch * ((a.M + 1) / 2 * 2) * a.N : 0;
+}
+
 }  // namespace
+
+size_t dgemm_scratch(const GemmArgs& a) {
+  if (a.M <= 0 || a.N <= 0 || a.batch <= 0 || !long_k(a)) return 0;
+  return scratch_elems(a, plan_gemm(a, num_sms()));
+}
 
 int num_sms() {
   static std::atomic<int> cache[kMaxDevices];
@@ -463,7 +563,7 @@ int num_sms() {
   });
 }
 
-cudaError_t dgemm(GemmArgs a, cudaStream_t st) {
+cudaError_t dgemm(GemmArgs a, cudaStream_t st, double* scratch) {
   if (a.M <= 0 || a.N <= 0 || a.batch <= 0) return cudaSuccess;
   if (a.tri && a.M != a.N) return cudaErrorInvalidValue;
   // 16-byte cp.async path when every tile chunk is 16-byte aligned, else 8-byte copies
@@ -482,12 +582,17 @@ cudaError_t dgemm(GemmArgs a, cudaStream_t st) {
   }
   KParams kp;
   kp.g = a;
-  const int cfg = pick_cfg(a);
+  Plan plan = plan_gemm(a, sms);
+  if (plan.groups > 1 && !scratch) plan = Plan{plan.cfg, plan.cluster, 1};
+  const int cfg = plan.cfg;
   int BM, BN, per_sm;
   tile_dims(cfg, &BM, &BN, &per_sm);
   kp.tiles_m = (a.M + BM - 1) / BM;
   kp.tiles_n = (a.N + BN - 1) / BN;
-  kp.splitk = choose_splitk(a, sms);
+  kp.splitk = plan.cluster * plan.groups;
+  kp.cluster = plan.cluster;
+  kp.P = scratch;
+  kp.ldp = (a.M + 1) / 2 * 2;
   kp.stage_c = (kp.splitk <= 1 && a.beta != 0.0 && !a.tri && !a.kto_m && !a.alpha_vec &&
                  (a.alpha == 1.0 || a.alpha == -1.0) && (a.K <= 64 || (cfg == 2 && a.K <= 256)))
                    ? 1
@@ -500,7 +605,10 @@ cudaError_t dgemm(GemmArgs a, cudaStream_t st) {
                         : cfg == 2 ? launch_c<CfgSmall>(kp, grid, v16, st)
                         : cfg == 4 ? launch_c<CfgTiny>(kp, grid, v16, st)
                                    : launch_c<CfgWide>(kp, grid, v16, st);
-  return e;
+  if (e != cudaSuccess || plan.groups <= 1) return e;
+  const int blocks = static_cast<int>(std::min<int64_t>((static_cast<int64_t>(a.M) * a.N + 255) / 256, 4 * sms));
+  return launch_dependent(splitk_reduce_kernel, dim3(blocks, a.batch), dim3(256), 0, st, dim3(1), a, plan.groups,
+                          scratch, kp.ldp);
 }
 
 }  // namespace zolo

@@ -29,7 +29,10 @@ struct GemmArgs {
   int splitk = 0;   // 0 = choose; 1 = off; >1 = number of K slices
 };
 
-cudaError_t dgemm(GemmArgs a, cudaStream_t st);
+// scratch: dgemm_scratch(a) doubles on the device, used by this launch's stream alone until it is done, or null
+// (a long K over few tiles is then split less).
+cudaError_t dgemm(GemmArgs a, cudaStream_t st, double* scratch = nullptr);
+size_t dgemm_scratch(const GemmArgs& a);
 // Streaming rank-k update C = beta*C + alpha*A*B (no transposes, K <= 32; update.cu).
 // dgemm dispatches to it when rank_update_applies(a).
 bool rank_update_applies(const GemmArgs& a);

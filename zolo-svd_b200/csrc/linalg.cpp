@@ -105,9 +105,12 @@ void gemm(Context& c, int transA, int transB, int M, int N, int K, double alpha,
     const double f = algo_flops(M, N, K, tri, kfrom_n, kto_m);
     c.prof.begin(cls, f * batch, s, &rec);
   }
-  ck(dgemm(a, s));
+  const size_t need = dgemm_scratch(a);
+  // one buffer a stream: the products of a stream follow one another
+  double* scratch = need ? c.buf(s == c.stream() ? "gemm_k" : "gemm_k_side", need) : nullptr;
+  ck(dgemm(a, s, scratch));
   if (c.prof.on) c.prof.end(rec, s);
-  c.stats.launches++;
+  c.stats.launches += need ? 2 : 1;
 }
 
 void ozgemm(Context& c, int transA, int transB, int M, int N, int K, double alpha, Mat A, Mat B, double beta, Mat C,
