@@ -49,3 +49,23 @@ def test_one_step_again(m, n, kappa):
     again = _qdwh(h, a, m, n, 0)
     h.close()
     assert np.array_equal(again[0], q0) and np.array_equal(again[1], h0)
+
+
+def test_bound_past_one():
+    """The lower bound of a single column is 1 up to rounding; past 1 it has no weights (not a number), and the
+    iteration ends after its first step as at any other converged L."""
+    import torch
+    hd = zb.Handle(0)
+    rng = np.random.default_rng(5)
+    past = 0
+    for _ in range(24):
+        a = rng.standard_normal((2, 1))
+        da = zb.colmajor_to_device(a)
+        dq, dh = torch.zeros_like(da), torch.zeros((1, 1), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        assert zb.qdwh_dev(hd, "N", 2, 1, 0.0, da.data_ptr(), 2, dq.data_ptr(), 2, dh.data_ptr(), 1, 0, 12, 0) == 0
+        st = hd.stats()
+        past += st["beta"] > 1.0
+        assert st["iterations"] == 1
+    hd.close()
+    assert past > 0

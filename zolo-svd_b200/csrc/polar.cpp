@@ -521,7 +521,7 @@ int qdwh(Context& c, int m, int n, const double* dA, int64_t lda, double* dQ, in
   int it = 0, failed = -1, first_chol = kMaxSteps;
   while (true) {
     const bool over = (o.maxit >= 0 && it > o.maxit) || it >= kMaxSteps;
-    const bool converged = std::fabs(1.0 - lowk) <= tol1;
+    const bool converged = !(std::fabs(1.0 - lowk) > tol1);  // an L that is not a number too
     if (it > 0 && (over || converged)) {
       const int k = read_back(it);
       if (k >= 0) {
@@ -547,7 +547,7 @@ int qdwh(Context& c, int m, int n, const double* dA, int64_t lda, double* dQ, in
     qdwh_weights(lowk, &ak, &bk, &ckk, &lnext);
     lowk = lnext;
     double akk, bkk;
-    if (ckk <= 100.0 && it != failed) {
+    if (!(ckk > 100.0) && it != failed) {
       before[it].chol = true;
       first_chol = std::min(first_chol, it);
       OzScope mixed_ch(c, c.zolo_mixed >= 1);  // the mixed form's products of this Cholesky step
