@@ -117,12 +117,13 @@ int zolo_profile_read(zolo_handle_t handle, double* out, int reset);
  * measured check rather than on ||X_{k+1} - X_k||.  No reference counterpart. */
 #define ZOLO_OPT_NS_FINISH 2
 /* ZOLO_OPT_CHOL_INVERSE: 0 (default) = each Cholesky-form term solves
- * X (X^T X + c_j I)^{-1} by L_j^{-T} and then L_j^{-1} (zolochol.f90:87-113); 1 = the
- * terms' inverses L_j^{-T} L_j^{-1} (triangular inverse + one lower-triangle product,
- * 4n^3/3 per term) are summed into S = sum_j w_j (X^T X + c_j I)^{-1} and the iteration
- * takes one Z = X S, about 6n^3 fewer flops per iteration for r = 8.  These matrices
- * are well conditioned in the Cholesky iterations (condition <= CON^2, CON <= 1e3), so
- * both forms agree to rounding.  SYM = 'S' keeps the two factors.  No reference counterpart. */
+ * X (X^T X + c_j I)^{-1} by L_j^{-T} and then L_j^{-1} (zolochol.f90:87-113), as products up to
+ * CON = 12 and by substitution above; 1 = the terms' inverses L_j^{-T} L_j^{-1} (triangular
+ * inverse + one lower-triangle product, 4n^3/3 per term) are summed into
+ * S = sum_j w_j (X^T X + c_j I)^{-1} and the iteration takes one Z = X S, about 6n^3 fewer flops
+ * per iteration for r = 8.  These matrices have condition <= CON^2 in the Cholesky iterations
+ * (CON <= 1e3); the sum form's error grows with CON, and with ZOLO_OPT_TERM_PLAN it starts at
+ * CON <= 12, where both agree to rounding.  SYM = 'S' keeps the two factors.  No reference counterpart. */
 #define ZOLO_OPT_CHOL_INVERSE 3
 /* ZOLO_OPT_BETA_FROB: 0 (default) = zolo_polar_dev takes beta = 1/(sqrt(n) ||R^{-1}||_1)
  * (zolo_bounds_dev mode 1, the reference driver's estimate); 1 = beta = 1/||R^{-1}||_F (mode 2),

@@ -7,7 +7,7 @@ stream).  The cases are the shapes that dominate a Zolo-PD / QDWH solve, so a
 profiler pointed at one case sees the same kernel configuration as the full
 solve (e.g. ``ncu -k regex:dgemm_kernel ... python kernel_cases.py --case gemm_nn``):
 
-  gemm_nn      C = A B, M = N = K = n          (general DMMA GEMM, 128 x 128 tiles)
+  gemm_nn      C = A B, M = N = K = n          (general DMMA GEMM, 64 x 64 tiles)
   gemm_rank32  C -= A B, M = N = n, K = 32     (streaming rank-32 update kernel)
   gemm_k128    C -= A B, M = N = n, K = 128    (block-reflector update, 64 x 64 tiles, C staged)
   gemm_m32     P = V^T W, M = 32, N = K = n    (panel projection, 32 x 64 tiles)

@@ -98,8 +98,8 @@ class Context {
   int zolo_shared_qr = 1;
   // Zolo-PD stopping: 0 = reference rule, 1 = Newton-Schulz finish once ||X^T X - I|| is small.
   int zolo_ns_finish = 0;
-  // Zolo-PD Cholesky iterations: 0 = two products with L^-T and L^-1 per term (zolochol.f90),
-  // 1 = explicit inverses summed into S, then one Z = X S.
+  // Zolo-PD Cholesky iterations: 0 = L^-T and then L^-1 per term (zolochol.f90; by
+  // products up to CON = 12, else by substitution), 1 = explicit inverses summed into S, then one Z = X S.
   int zolo_chol_inverse = 0;
   // zolo_polar's bounds: 0 = beta = 1/(sqrt(n) ||R^-1||_1) (test_zolodrv1.f90), 1 = 1/||R^-1||_F.
   int zolo_beta_frob = 0;

@@ -748,7 +748,7 @@ __global__ void extract_v_kernel(int m, int w, const double* A, int64_t lda, int
 // T12 = -T1 (V1^T V2) T2 for pairs of 32 columns, then of 64, in one CTA's shared memory (both
 // products on the FP64 tensor path).  One array holds T in its upper triangle and V^T V strictly below the
 // panels' diagonal blocks.  blockIdx.x: the 128-column block of TB; the CTA writes its columns, zero
-// outside its own rows.  Bound by latency: 7 us (25 with the loads in eight dependent rounds), where the
+// outside its own rows.  Bound by latency: 9 us (25 with the loads in eight dependent rounds), where the
 // set-up and six small products of the panel-by-panel recursion were a chain of 30 us.
 constexpr int BTW = 128, BTT = 512;
 constexpr int BTL = BTW + 4, BTP = 64 + 4;  // = 4 mod 16: conflict-free fragment loads
